@@ -170,15 +170,28 @@ struct icf_contact_ws {
 
 // Device MINRES solver state (icf_solve.cu).
 struct icf_solver {
-  long long gen = -1;  // structure generation the lower-block index belongs to
-  int *lrows = nullptr, *lcols = nullptr, *lslot = nullptr;
-  long long rows_cap = 0, l_cap = 0, ls_cap = 0;
-  double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *dinv = nullptr;
-  double *w = nullptr, *w2 = nullptr;
-  long long x_cap = 0, r_cap = 0, z_cap = 0, p_cap = 0, q_cap = 0, d_cap = 0, w_cap = 0, w2_cap = 0;
-  double *part = nullptr, *sc = nullptr;
-  double *h_sc = nullptr;  // pinned
-  int n_indefinite = 0;    // diagonal blocks of the last solve preconditioned by |S|^-1
+  // row order (position -> row and back), of order_rows rows
+  int order_rows = -1;
+  int *perm = nullptr, *iperm = nullptr;
+  long long perm_cap = 0, iperm_cap = 0;
+  // of structure generation gen: the first step of every position, the
+  // entries of the steps and their marks, the warps' first positions and
+  // batches, the thread blocks' halos
+  long long gen = -1;
+  int *sstep = nullptr, *eslot = nullptr, *ecol = nullptr, *part = nullptr, *first = nullptr, *hcount = nullptr,
+      *hcol = nullptr;
+  unsigned short *eidx = nullptr;
+  unsigned char *last = nullptr;
+  long long sstep_cap = 0, eslot_cap = 0, ecol_cap = 0, eidx_cap = 0, last_cap = 0, n_steps = 0;
+  int blocks = 0;
+  bool halo = false;
+  int most[3] = {0, 0, 0};  // rows and halo of the largest thread block, batches of the largest warp
+  double *rec = nullptr, *x = nullptr, *vec = nullptr;  // the matrix's records; the solution; the iteration's vectors
+  long long rec_cap = 0, x_cap = 0, vec_cap = 0;
+  double *sc = nullptr, *h_sc = nullptr;  // scalars between launches, and pinned
+  unsigned long long *slots = nullptr;    // the grid-wide exchanges' words
+  unsigned epoch = 0;                     // exchanges numbered so far
+  int n_indefinite = 0;  // diagonal blocks of the last solve preconditioned by |S|^-1
 };
 
 // Parameters the kernels read, passed by value (they live in the kernel
