@@ -16,10 +16,10 @@
 // are rounded to bf16 before each product; biases, GELU and all sums are
 // FP32.
 //
-// Training: the forward above (keeping Z1, H1, Z2, H2), then the backward in
-// FP32 CUDA-core arithmetic, per-chunk weight-gradient partials and a fixed
-// order reduction (no atomics: a gradient is identical run to run), and Adam
-// on FP32 master weights, after which the bf16 copies are refreshed.
+// Training: forward, FP32 CUDA-core backward and weight-gradient partials of 32
+// nodes per block in one kernel, a fixed order reduction of the partials (no
+// atomics: a gradient is identical run to run), and Adam on FP32 master
+// weights, after which the bf16 copies are refreshed.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -53,14 +53,13 @@ struct icf_mlp {
   __nv_bfloat16 *d_wb = nullptr;  // bf16 weights, padded: W1 64x16, W2 64x64, W3 8x64
   float *d_norm = nullptr;        // in_shift[15], in_scale[15], out_scale[3]
   long long adam_t = 0;
-  // training buffers
-  int cap = 0;
-  float *d_x = nullptr, *d_y = nullptr;
-  float *d_z1 = nullptr, *d_h1 = nullptr, *d_z2 = nullptr, *d_h2 = nullptr, *d_out = nullptr;
-  float *d_dy = nullptr, *d_dz1 = nullptr, *d_dz2 = nullptr;
-  float *d_part = nullptr;  // per-chunk gradient partials
-  int part_cap = 0;
-  float *d_grad = nullptr, *d_loss = nullptr;
+  // inputs, outputs, targets (or output gradients), activations of
+  // forward_trace, gradient partials and losses, with their elements
+  float *d_x = nullptr, *d_out = nullptr, *d_y = nullptr;
+  float *d_z1 = nullptr, *d_h1 = nullptr, *d_z2 = nullptr, *d_h2 = nullptr;
+  float *d_part = nullptr, *d_loss = nullptr, *d_grad = nullptr;
+  long long x_cap = 0, out_cap = 0, y_cap = 0, z1_cap = 0, h1_cap = 0, z2_cap = 0, h2_cap = 0, part_cap = 0,
+            loss_cap = 0;
 };
 
 namespace {
@@ -201,14 +200,11 @@ __global__ void __launch_bounds__(256) k_mlp_infer(int n, const float *__restric
   }
 }
 
-// training forward: keeps Z1, H1 = bf16(GELU(Z1)), Z2, H2 and dY = 2 (y - t) / n
-// (mean squared error over nodes and components); loss partial per warp-tile
-__global__ void __launch_bounds__(256) k_mlp_fwd_train(int n, const float *__restrict__ x, const float *__restrict__ tgt,
-                                                       const __nv_bfloat16 *wb, const float *master,
-                                                       const float *norm, float *__restrict__ z1,
-                                                       float *__restrict__ h1, float *__restrict__ z2,
-                                                       float *__restrict__ h2, float *__restrict__ dy,
-                                                       float *__restrict__ loss_part) {
+// forward that keeps Z1, H1 = bf16(GELU(Z1)), Z2 and H2 (forward_trace)
+__global__ void __launch_bounds__(256) k_mlp_trace(int n, const float *__restrict__ x, const __nv_bfloat16 *wb,
+                                                   const float *master, const float *norm, float *__restrict__ z1,
+                                                   float *__restrict__ h1, float *__restrict__ z2,
+                                                   float *__restrict__ h2) {
   __shared__ __nv_bfloat16 sW[WB_N];
   __shared__ float sB[NPAR];
   __shared__ float sNorm[2 * NI + NO];
@@ -216,152 +212,270 @@ __global__ void __launch_bounds__(256) k_mlp_fwd_train(int n, const float *__res
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int r0 = 16 * warp;
-  float l = 0.f;
-  if (r0 < n) {
-    fwd_out f;
-    mlp_forward16(x, n, r0, sW, sB, sNorm, lane, f);
-    const int g = lane >> 2, t = lane & 3;
+  if (r0 >= n) return;
+  fwd_out f;
+  mlp_forward16(x, n, r0, sW, sB, sNorm, lane, f);
+  const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int j = 0; j < 8; j++)
+  for (int j = 0; j < 8; j++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int r = r0 + g + (e >= 2 ? 8 : 0), c = 8 * j + 2 * t + (e & 1);
+      if (r < n) {
+        z1[(size_t)r * NH + c] = f.z1[j][e];
+        h1[(size_t)r * NH + c] = bf16r(gelu(f.z1[j][e]));
+        z2[(size_t)r * NH + c] = f.z2[j][e];
+        h2[(size_t)r * NH + c] = bf16r(gelu(f.z2[j][e]));
+      }
+    }
+}
+
+// ---- gradient: forward, backward and weight gradients of 32 nodes per block -----
+// Everything of the 32 nodes stays in shared memory; a block writes only its
+// partial of every weight and bias gradient,
+//   dW1 = dZ1^T Xn, db1 = sum dZ1, dW2 = dZ2^T H1, db2 = sum dZ2,
+//   dW3 = dY^T H2, db3 = sum dY
+// (Xn the bf16-rounded normalised inputs), and of the loss.  The backward is
+// dZ2 = (dY W3) * gelu'(Z2), dZ1 = (dZ2 W2) * gelu'(Z1) with W the bf16 values,
+// FP32 throughout; the partials of NODES nodes, of CHUNK nodes and of all are
+// added in this order (k_mlp_reduce), so a gradient is identical run to run.
+//
+// What bounds it: at a training batch (4096 nodes, 128 blocks, one wave) the
+// chain of a block's phases.  As four kernels with the activations in global
+// memory, the weight gradients by one block per 1024 nodes (4 blocks, 262 us) and
+// the backward by one thread per node (32 blocks, 131 us), the batch took 424 us
+// on the device (437 us a call with its host copies); now 22 us and 7 us (91 us a
+// call, bound by the copies of the 295 KB batch from pageable memory).
+constexpr int NODES = 32;
+constexpr int CHUNK = 1024;  // nodes whose partials are added first
+constexpr int LDH = NH + 4;  // padded row of a node's hidden values
+
+struct grad_smem {
+  __nv_bfloat16 W[WB_N];
+  float W2[NH * NH];  // the bf16 values
+  float W3[NO * NH];
+  float B1[NH], B2[NH], B3[NO + 1];
+  float norm[2 * NI + 2];
+  float x[NODES][16];                    // normalised, rounded to bf16; column 15 zero
+  float z1[NODES][LDH], z2[NODES][LDH];  // pre-activations, later dZ1 and dZ2
+  float h1[NODES][LDH], h2[NODES][LDH];  // bf16 values
+  float dy[NODES][4];
+};
+
+// A fragment of 16 rows, columns 16 kk ..: bf16 values held as floats
+template <int LD>
+__device__ __forceinline__ void afrag(const float (*H)[LD], int r0, int kk, int lane, uint32_t a[4]) {
+  const int g = lane >> 2, t = lane & 3, c = 16 * kk + 2 * t;
+  a[0] = pack_bf16(H[r0 + g][c], H[r0 + g][c + 1]);
+  a[1] = pack_bf16(H[r0 + g + 8][c], H[r0 + g + 8][c + 1]);
+  a[2] = pack_bf16(H[r0 + g][c + 8], H[r0 + g][c + 9]);
+  a[3] = pack_bf16(H[r0 + g + 8][c + 8], H[r0 + g + 8][c + 9]);
+}
+
+// tgt: the loss is the mean squared error against it; tgt == nullptr: dyin is
+// dL/d(output)
+__global__ void __launch_bounds__(256) k_mlp_grad(int n, const float *__restrict__ x, const float *__restrict__ tgt,
+                                                  const float *__restrict__ dyin, const __nv_bfloat16 *wb,
+                                                  const float *master, const float *norm, float *__restrict__ part,
+                                                  float *__restrict__ loss_part) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  grad_smem &S = *reinterpret_cast<grad_smem *>(raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b0 = blockIdx.x * NODES;
+  for (int i = tid; i < WB_N / 2; i += 256) reinterpret_cast<uint32_t *>(S.W)[i] = reinterpret_cast<const uint32_t *>(wb)[i];
+  for (int i = tid; i < NH * NH; i += 256) S.W2[i] = __bfloat162float(wb[WB_W2 + i]);
+  for (int i = tid; i < NO * NH; i += 256) S.W3[i] = __bfloat162float(wb[WB_W3 + i]);
+  if (tid < NH) {
+    S.B1[tid] = master[OFF_B1 + tid];
+    S.B2[tid] = master[OFF_B2 + tid];
+  }
+  if (tid < NO) S.B3[tid] = master[OFF_B3 + tid];
+  for (int i = tid; i < NODES * 16; i += 256) {
+    const int r = i / 16, c = i % 16;
+    S.x[r][c] = b0 + r < n && c < NI ? bf16r((x[(size_t)(b0 + r) * NI + c] - norm[c]) * norm[NI + c]) : 0.f;
+  }
+  __syncthreads();
+  // layers 1 and 2: warp w computes the hidden units 8 w .. 8 w + 7 of all nodes
+  const int g = lane >> 2, t = lane & 3, c0 = 8 * warp + 2 * t;
+#pragma unroll
+  for (int layer = 1; layer <= 2; layer++) {
+    float (*Z)[LDH] = layer == 1 ? S.z1 : S.z2, (*H)[LDH] = layer == 1 ? S.h1 : S.h2;
+    const float bb0 = layer == 1 ? S.B1[c0] : S.B2[c0], bb1 = layer == 1 ? S.B1[c0 + 1] : S.B2[c0 + 1];
+#pragma unroll
+    for (int r0 = 0; r0 < NODES; r0 += 16) {
+      float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < (layer == 1 ? 1 : 4); kk++) {
+        uint32_t a[4], b[2];
+        if (layer == 1) {
+          afrag(S.x, r0, 0, lane, a);
+          bfrag(S.W + WB_W1, 16, warp, 0, lane, b);
+        } else {
+          afrag(S.h1, r0, kk, lane, a);
+          bfrag(S.W + WB_W2, NH, warp, kk, lane, b);
+        }
+        mma_bf16(z, a, b);
+      }
+      z[0] += bb0; z[1] += bb1; z[2] += bb0; z[3] += bb1;
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        const int r = r0 + g + (e >= 2 ? 8 : 0), c = 8 * j + 2 * t + (e & 1);
-        if (r < n) {
-          z1[(size_t)r * NH + c] = f.z1[j][e];
-          h1[(size_t)r * NH + c] = bf16r(gelu(f.z1[j][e]));
-          z2[(size_t)r * NH + c] = f.z2[j][e];
-          h2[(size_t)r * NH + c] = bf16r(gelu(f.z2[j][e]));
-        }
+        const int r = r0 + g + (e >= 2 ? 8 : 0), c = c0 + (e & 1);
+        const bool ok = b0 + r < n;
+        Z[r][c] = z[e];
+        H[r][c] = ok ? bf16r(gelu(z[e])) : 0.f;
       }
-    const float inv = 2.0f / (float)(n * NO);
-    if (tgt != nullptr) {  // tgt == nullptr: dy was supplied by the caller
+    }
+    __syncthreads();
+  }
+  // layer 3, its error and loss: one warp per 16 nodes
+  if (warp < NODES / 16) {
+    const int r0 = 16 * warp;
+    float l = 0.f;
+    if (tgt != nullptr) {
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++) {
+        uint32_t a[4], b[2];
+        afrag(S.h2, r0, kk, lane, a);
+        bfrag(S.W + WB_W3, NH, 0, kk, lane, b);
+        mma_bf16(y, a, b);
+      }
+      const float inv = 2.0f / (float)(n * NO);
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int r = r0 + g + (e >= 2 ? 8 : 0), c = 2 * t + (e & 1);
-        if (r < n && c < NO) {
-          const float d = f.y[e] - tgt[(size_t)r * NO + c];
-          dy[(size_t)r * NO + c] = inv * d;
+        if (c >= NO) continue;
+        float v = 0.f;
+        if (b0 + r < n) {
+          const float d = (y[e] + S.B3[c]) - tgt[(size_t)(b0 + r) * NO + c];
+          v = inv * d;
           l += d * d;
         }
+        S.dy[r][c] = v;
+      }
+    } else {
+      for (int i = lane; i < 16 * NO; i += 32) {
+        const int r = r0 + i / NO, c = i % NO;
+        S.dy[r][c] = b0 + r < n ? dyin[(size_t)(b0 + r) * NO + c] : 0.f;
       }
     }
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+    if (lane == 0) loss_part[(NODES / 16) * blockIdx.x + warp] = l;
   }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-  if (lane == 0) loss_part[warp] = l;
-}
-
-// backward through the activations, one thread per node:
-// dZ2 = (dY W3) * gelu'(Z2);  dZ1 = (dZ2 W2) * gelu'(Z1)   (W = bf16 values)
-__global__ void __launch_bounds__(128) k_mlp_bwd_act(int n, const __nv_bfloat16 *wb, const float *__restrict__ z1,
-                                                     const float *__restrict__ z2, const float *__restrict__ dy,
-                                                     float *__restrict__ dz1, float *__restrict__ dz2) {
-  __shared__ float sW2[NH * NH];
-  __shared__ float sW3[NO * NH];
-  for (int i = threadIdx.x; i < NH * NH; i += blockDim.x) sW2[i] = __bfloat162float(wb[WB_W2 + i]);
-  for (int i = threadIdx.x; i < NO * NH; i += blockDim.x) sW3[i] = __bfloat162float(wb[WB_W3 + i]);
   __syncthreads();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const float d0 = dy[(size_t)r * NO], d1 = dy[(size_t)r * NO + 1], d2 = dy[(size_t)r * NO + 2];
-  float g2[NH];
-#pragma unroll 8
-  for (int j = 0; j < NH; j++) {
-    const float dh = d0 * sW3[j] + d1 * sW3[NH + j] + d2 * sW3[2 * NH + j];
-    g2[j] = dh * gelu_d(z2[(size_t)r * NH + j]);
-    dz2[(size_t)r * NH + j] = g2[j];
+  // dZ2 in place of Z2
+  for (int i = tid; i < NODES * NH; i += 256) {
+    const int r = i / NH, j = i % NH;
+    const float dh = S.dy[r][0] * S.W3[j] + S.dy[r][1] * S.W3[NH + j] + S.dy[r][2] * S.W3[2 * NH + j];
+    S.z2[r][j] = b0 + r < n ? dh * gelu_d(S.z2[r][j]) : 0.f;
   }
-  for (int i = 0; i < NH; i++) {
-    float dh = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < NH; j++) dh += g2[j] * sW2[j * NH + i];
-    dz1[(size_t)r * NH + i] = dh * gelu_d(z1[(size_t)r * NH + i]);
+  __syncthreads();
+  // dZ1 in place of Z1: eight units of one node per thread
+  {
+    const int r = tid / 8, i0 = 8 * (tid % 8);
+    float dh[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int j = 0; j < NH; j++) {
+      const float d = S.z2[r][j];
+      const float4 wa = *reinterpret_cast<const float4 *>(S.W2 + NH * j + i0);
+      const float4 wc = *reinterpret_cast<const float4 *>(S.W2 + NH * j + i0 + 4);
+      dh[0] += d * wa.x; dh[1] += d * wa.y; dh[2] += d * wa.z; dh[3] += d * wa.w;
+      dh[4] += d * wc.x; dh[5] += d * wc.y; dh[6] += d * wc.z; dh[7] += d * wc.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) S.z1[r][i0 + k] = b0 + r < n ? dh[k] * gelu_d(S.z1[r][i0 + k]) : 0.f;
   }
-}
-
-constexpr int CHUNK = 1024;  // nodes per weight-gradient partial
-
-// Partials of every weight and bias gradient over one chunk of nodes:
-//   dW1 = dZ1^T Xn, db1 = sum dZ1, dW2 = dZ2^T H1, db2 = sum dZ2,
-//   dW3 = dY^T H2, db3 = sum dY
-// (Xn the bf16-rounded normalised inputs).  256 threads; thread i owns
-// parameters i, i + 256, ... and walks the chunk in order.
-__global__ void __launch_bounds__(256) k_mlp_wgrad(int n, const float *__restrict__ x, const float *norm,
-                                                   const float *__restrict__ h1, const float *__restrict__ h2,
-                                                   const float *__restrict__ dz1, const float *__restrict__ dz2,
-                                                   const float *__restrict__ dy, float *__restrict__ part) {
-  __shared__ float sx[32][NI], sh1[32][NH], sh2[32][NH], sg1[32][NH], sg2[32][NH], sdy[32][NO];
-  constexpr int PER = (NPAR + 255) / 256;
-  float acc[PER];
+  __syncthreads();
+  // the partials: a 4 x 4 tile of dW2 per thread, four inputs of a unit of dW1,
+  // then dW3 and the biases
+  float *P = part + (size_t)blockIdx.x * NPAR;
+  {
+    const int o0 = 4 * (tid / 16), i0 = 4 * (tid % 16);
+    float a[4][4], bs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int q = 0; q < PER; q++) acc[q] = 0.f;
-  const int b0 = blockIdx.x * CHUNK, b1 = min(n, b0 + CHUNK);
-  for (int s0 = b0; s0 < b1; s0 += 32) {
-    const int m = min(32, b1 - s0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < 32 * NH; i += blockDim.x) {
-      const int r = i / NH, c = i % NH;
-      const bool ok = r < m;
-      sh1[r][c] = ok ? h1[(size_t)(s0 + r) * NH + c] : 0.f;
-      sh2[r][c] = ok ? h2[(size_t)(s0 + r) * NH + c] : 0.f;
-      sg1[r][c] = ok ? dz1[(size_t)(s0 + r) * NH + c] : 0.f;
-      sg2[r][c] = ok ? dz2[(size_t)(s0 + r) * NH + c] : 0.f;
-    }
-    for (int i = threadIdx.x; i < 32 * NI; i += blockDim.x) {
-      const int r = i / NI, c = i % NI;
-      sx[r][c] = r < m ? bf16r((x[(size_t)(s0 + r) * NI + c] - norm[c]) * norm[NI + c]) : 0.f;
-    }
-    for (int i = threadIdx.x; i < 32 * NO; i += blockDim.x) {
-      const int r = i / NO, c = i % NO;
-      sdy[r][c] = r < m ? dy[(size_t)(s0 + r) * NO + c] : 0.f;
-    }
-    __syncthreads();
+    for (int p = 0; p < 4; p++)
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-      const int p = threadIdx.x + 256 * q;
-      if (p >= NPAR) break;
-      float s = 0.f;
-      if (p < OFF_B1) {
-        const int o = p / NI, i = p % NI;
-        for (int r = 0; r < 32; r++) s += sg1[r][o] * sx[r][i];
-      } else if (p < OFF_W2) {
-        const int o = p - OFF_B1;
-        for (int r = 0; r < 32; r++) s += sg1[r][o];
-      } else if (p < OFF_B2) {
-        const int o = (p - OFF_W2) / NH, i = (p - OFF_W2) % NH;
-        for (int r = 0; r < 32; r++) s += sg2[r][o] * sh1[r][i];
-      } else if (p < OFF_W3) {
-        const int o = p - OFF_B2;
-        for (int r = 0; r < 32; r++) s += sg2[r][o];
-      } else if (p < OFF_B3) {
-        const int o = (p - OFF_W3) / NH, i = (p - OFF_W3) % NH;
-        for (int r = 0; r < 32; r++) s += sdy[r][o] * sh2[r][i];
-      } else {
-        const int o = p - OFF_B3;
-        for (int r = 0; r < 32; r++) s += sdy[r][o];
+      for (int q = 0; q < 4; q++) a[p][q] = 0.f;
+#pragma unroll 4
+    for (int r = 0; r < NODES; r++) {
+      const float4 d = *reinterpret_cast<const float4 *>(&S.z2[r][o0]), h = *reinterpret_cast<const float4 *>(&S.h1[r][i0]);
+      const float dv[4] = {d.x, d.y, d.z, d.w}, hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        bs[p] += dv[p];
+#pragma unroll
+        for (int q = 0; q < 4; q++) a[p][q] += dv[p] * hv[q];
       }
-      acc[q] += s;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) P[OFF_W2 + NH * (o0 + p) + i0 + q] = a[p][q];
+      if (i0 == 0) P[OFF_B2 + o0 + p] = bs[p];
     }
   }
+  {
+    const int o = tid / 4, i0 = 4 * (tid % 4);
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, bs = 0.f;
+#pragma unroll 4
+    for (int r = 0; r < NODES; r++) {
+      const float d = S.z1[r][o];
+      const float4 v = *reinterpret_cast<const float4 *>(&S.x[r][i0]);
+      a[0] += d * v.x; a[1] += d * v.y; a[2] += d * v.z; a[3] += d * v.w;
+      bs += d;
+    }
 #pragma unroll
-  for (int q = 0; q < PER; q++) {
-    const int p = threadIdx.x + 256 * q;
-    if (p < NPAR) part[(size_t)blockIdx.x * NPAR + p] = acc[q];
+    for (int k = 0; k < 4; k++)
+      if (i0 + k < NI) P[OFF_W1 + NI * o + i0 + k] = a[k];
+    if (i0 == 0) P[OFF_B1 + o] = bs;
+  }
+  if (tid < NO * NH) {
+    const int o = tid / NH, i = tid % NH;
+    float a = 0.f;
+    for (int r = 0; r < NODES; r++) a += S.dy[r][o] * S.h2[r][i];
+    P[OFF_W3 + tid] = a;
+  } else if (tid < NO * NH + NO) {
+    float a = 0.f;
+    for (int r = 0; r < NODES; r++) a += S.dy[r][tid - NO * NH];
+    P[OFF_B3 + tid - NO * NH] = a;
   }
 }
 
-// grad[p] = sum over chunks in order; loss = sum of warp partials / (n NO)
-__global__ void k_mlp_reduce(int nchunks, const float *__restrict__ part, float *__restrict__ grad, int nloss,
-                             const float *__restrict__ loss_part, float *loss, int n) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < NPAR) {
-    float s = 0.f;
-    for (int c = 0; c < nchunks; c++) s += part[(size_t)c * NPAR + p];
-    grad[p] = s;
+// grad[p]: the partials of every CHUNK nodes in order, then the chunks in order
+// (32 parameters per block, eight chunks side by side); loss = sum of its
+// partials in order / (n NO)
+__global__ void __launch_bounds__(256) k_mlp_reduce(int nparts, const float *__restrict__ part, float *__restrict__ grad,
+                                                    int nloss, const float *__restrict__ loss_part, float *loss, int n) {
+  constexpr int PER = CHUNK / NODES;
+  __shared__ float sh[8][32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, p = 32 * blockIdx.x + tx;
+  const int nch = (nparts + PER - 1) / PER;
+  float s = 0.f;
+  for (int c0 = 0; c0 < nch; c0 += 8) {
+    float a = 0.f;
+    if (p < NPAR) {
+      const int q0 = (c0 + ty) * PER, q1 = min(nparts, q0 + PER);
+#pragma unroll 8
+      for (int q = q0; q < q1; q++) a += part[(size_t)q * NPAR + p];
+    }
+    sh[ty][tx] = a;
+    __syncthreads();
+    if (ty == 0)
+      for (int k = 0; k < 8 && c0 + k < nch; k++) s += sh[k][tx];
+    __syncthreads();
   }
-  if (p == 0 && loss) {
+  if (ty == 0 && p < NPAR) grad[p] = s;
+  if (blockIdx.x == 0 && loss) {
+    __shared__ float sl[256];
     float l = 0.f;
-    for (int i = 0; i < nloss; i++) l += loss_part[i];
-    *loss = l / (float)(n * NO);
+    for (int i0 = 0; i0 < nloss; i0 += 256) {
+      sl[threadIdx.x] = i0 + (int)threadIdx.x < nloss ? loss_part[i0 + threadIdx.x] : 0.f;
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (int i = 0; i < min(256, nloss - i0); i++) l += sl[i];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = l / (float)(n * NO);
   }
 }
 
@@ -412,43 +526,42 @@ int fail(icf_mlp *m, int code, const std::string &msg) {
     if (e_ != cudaSuccess) return fail((m), ICF_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-int ensure_cap(icf_mlp *m, int n) {
-  if (n <= m->cap) return ICF_OK;
-  float **bufs[] = {&m->d_x, &m->d_y, &m->d_z1, &m->d_h1, &m->d_z2, &m->d_h2, &m->d_out, &m->d_dy, &m->d_dz1, &m->d_dz2};
-  const size_t w[] = {NI, NO, NH, NH, NH, NH, NO, NO, NH, NH};
-  for (int i = 0; i < 10; i++) {
-    cudaFree(*bufs[i]);
-    *bufs[i] = nullptr;
-  }
-  for (int i = 0; i < 10; i++) MLP_CUDA(m, cudaMalloc(bufs[i], sizeof(float) * w[i] * (size_t)n));
-  m->cap = n;
-  const int nch = (n + CHUNK - 1) / CHUNK;
-  if (nch > m->part_cap) {
-    cudaFree(m->d_part);
-    m->d_part = nullptr;
-    MLP_CUDA(m, cudaMalloc(&m->d_part, sizeof(float) * NPAR * (size_t)nch));
-    m->part_cap = nch;
-  }
-  cudaFree(m->d_loss);
-  m->d_loss = nullptr;
-  MLP_CUDA(m, cudaMalloc(&m->d_loss, sizeof(float) * ((size_t)(n + 15) / 16 + 16)));
+// device arrays of at least n elements
+int ensure(icf_mlp *m, float **p, long long *cap, long long n) {
+  if (n <= *cap && *p) return ICF_OK;
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+  MLP_CUDA(m, cudaMalloc(p, sizeof(float) * (size_t)n));
+  *cap = n;
   return ICF_OK;
 }
 
-// forward + backward of the data already in d_x, d_y (n nodes): d_grad, loss.
-// dy_given: d_dy already holds dL/dy (the caller's loss), d_y is unused.
+// the inputs and outputs of n nodes
+int ensure_io(icf_mlp *m, long long n) {
+  if (ensure(m, &m->d_x, &m->x_cap, NI * n) || ensure(m, &m->d_out, &m->out_cap, NO * n)) return ICF_ERR_CUDA;
+  return ICF_OK;
+}
+// ... and their targets (or output gradients) and the gradient's partials
+int ensure_grad(icf_mlp *m, long long n) {
+  const long long nb = (n + NODES - 1) / NODES;
+  if (ensure(m, &m->d_x, &m->x_cap, NI * n) || ensure(m, &m->d_y, &m->y_cap, NO * n) ||
+      ensure(m, &m->d_part, &m->part_cap, NPAR * nb) || ensure(m, &m->d_loss, &m->loss_cap, 1 + (NODES / 16) * nb))
+    return ICF_ERR_CUDA;
+  return ICF_OK;
+}
+
+// gradient of the data already in d_x, d_y (n nodes): d_grad, loss.
+// dy_given: d_y holds dL/dy (the caller's loss) instead of targets.
 int grad_on_device(icf_mlp *m, int n, float *loss_host, bool dy_given = false) {
   cudaStream_t s = m->stream;
-  const int tiles = (n + 15) / 16;
-  const int blocks = (tiles + 7) / 8;
+  const int nb = (n + NODES - 1) / NODES;
   float *loss_part = m->d_loss + 1;
-  k_mlp_fwd_train<<<blocks, 256, 0, s>>>(n, m->d_x, dy_given ? nullptr : m->d_y, m->d_wb, m->d_master, m->d_norm,
-                                          m->d_z1, m->d_h1, m->d_z2, m->d_h2, m->d_dy, loss_part);
-  // warps beyond the last tile wrote zero partials: count them in
-  k_mlp_bwd_act<<<icf_blocks(n, 128), 128, 0, s>>>(n, m->d_wb, m->d_z1, m->d_z2, m->d_dy, m->d_dz1, m->d_dz2);
-  const int nch = (n + CHUNK - 1) / CHUNK;
-  k_mlp_wgrad<<<nch, 256, 0, s>>>(n, m->d_x, m->d_norm, m->d_h1, m->d_h2, m->d_dz1, m->d_dz2, m->d_dy, m->d_part);
-  k_mlp_reduce<<<icf_blocks(NPAR, 256), 256, 0, s>>>(nch, m->d_part, m->d_grad, blocks * 8, loss_part, m->d_loss, n);
+  MLP_CUDA(m, cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(grad_smem)));
+  k_mlp_grad<<<nb, 256, sizeof(grad_smem), s>>>(n, m->d_x, dy_given ? nullptr : m->d_y, m->d_y, m->d_wb, m->d_master,
+                                               m->d_norm, m->d_part, loss_part);
+  k_mlp_reduce<<<icf_blocks(NPAR, 32), 256, 0, s>>>(nb, m->d_part, m->d_grad, (NODES / 16) * nb, loss_part, m->d_loss,
+                                                   n);
   MLP_CUDA(m, cudaGetLastError());
   if (loss_host) {
     MLP_CUDA(m, cudaMemcpyAsync(loss_host, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -496,7 +609,7 @@ int icf_mlp_destroy(icf_mlp *m) {
   if (!m) return ICF_ERR_ARG;
   cudaSetDevice(m->device);
   void *p[] = {m->d_master, m->d_m, m->d_v, m->d_wb, m->d_norm, m->d_x, m->d_y, m->d_z1, m->d_h1, m->d_z2,
-               m->d_h2, m->d_out, m->d_dy, m->d_dz1, m->d_dz2, m->d_part, m->d_grad, m->d_loss};
+               m->d_h2, m->d_out, m->d_part, m->d_grad, m->d_loss};
   for (void *q : p) cudaFree(q);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
@@ -532,7 +645,7 @@ int icf_mlp_forward(icf_mlp *m, int n, const float *x, float *y) {
   if (!m || n < 0 || (n && (!x || !y))) return ICF_ERR_ARG;
   if (n == 0) return ICF_OK;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if (ensure_cap(m, n)) return ICF_ERR_CUDA;
+  if (ensure_io(m, n)) return ICF_ERR_CUDA;
   cudaStream_t s = m->stream;
   MLP_CUDA(m, cudaMemcpyAsync(m->d_x, x, sizeof(float) * NI * (size_t)n, cudaMemcpyHostToDevice, s));
   const int tiles = (n + 15) / 16;
@@ -548,13 +661,15 @@ int icf_mlp_forward(icf_mlp *m, int n, const float *x, float *y) {
 int icf_mlp_forward_trace(icf_mlp *m, int n, const float *x, float *z1, float *h1, float *z2, float *h2, float *y) {
   if (!m || n <= 0 || !x || !z1 || !h1 || !z2 || !h2 || !y) return ICF_ERR_ARG;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if (ensure_cap(m, n)) return ICF_ERR_CUDA;
+  const long long nz = (long long)NH * n;
+  if (ensure_io(m, n) || ensure(m, &m->d_z1, &m->z1_cap, nz) || ensure(m, &m->d_h1, &m->h1_cap, nz) ||
+      ensure(m, &m->d_z2, &m->z2_cap, nz) || ensure(m, &m->d_h2, &m->h2_cap, nz))
+    return ICF_ERR_CUDA;
   cudaStream_t s = m->stream;
   MLP_CUDA(m, cudaMemcpyAsync(m->d_x, x, sizeof(float) * NI * (size_t)n, cudaMemcpyHostToDevice, s));
   const int tiles = (n + 15) / 16;
-  // the training forward writes the activations (no target: dy untouched)
-  k_mlp_fwd_train<<<(tiles + 7) / 8, 256, 0, s>>>(n, m->d_x, nullptr, m->d_wb, m->d_master, m->d_norm, m->d_z1,
-                                                  m->d_h1, m->d_z2, m->d_h2, m->d_dy, m->d_loss + 1);
+  k_mlp_trace<<<(tiles + 7) / 8, 256, 0, s>>>(n, m->d_x, m->d_wb, m->d_master, m->d_norm, m->d_z1, m->d_h1, m->d_z2,
+                                              m->d_h2);
   int blocks = (tiles + 7) / 8;
   if (blocks > 1184) blocks = 1184;
   k_mlp_infer<<<blocks, 256, 0, s>>>(n, m->d_x, m->d_wb, m->d_master, m->d_norm, m->d_out);
@@ -572,24 +687,24 @@ int icf_mlp_forward_trace(icf_mlp *m, int n, const float *x, float *z1, float *h
 int icf_mlp_grad(icf_mlp *m, int n, const float *x, const float *y, float *grad, float *loss) {
   if (!m || n <= 0 || !x || !y || !grad) return ICF_ERR_ARG;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if (ensure_cap(m, n)) return ICF_ERR_CUDA;
+  if (ensure_grad(m, n)) return ICF_ERR_CUDA;
   cudaStream_t s = m->stream;
   MLP_CUDA(m, cudaMemcpyAsync(m->d_x, x, sizeof(float) * NI * (size_t)n, cudaMemcpyHostToDevice, s));
   MLP_CUDA(m, cudaMemcpyAsync(m->d_y, y, sizeof(float) * NO * (size_t)n, cudaMemcpyHostToDevice, s));
-  float l = 0.f;
-  if (grad_on_device(m, n, &l)) return ICF_ERR_CUDA;
-  MLP_CUDA(m, cudaMemcpy(grad, m->d_grad, sizeof(float) * NPAR, cudaMemcpyDeviceToHost));
-  if (loss) *loss = l;
+  if (grad_on_device(m, n, nullptr)) return ICF_ERR_CUDA;
+  MLP_CUDA(m, cudaMemcpyAsync(grad, m->d_grad, sizeof(float) * NPAR, cudaMemcpyDeviceToHost, s));
+  if (loss) MLP_CUDA(m, cudaMemcpyAsync(loss, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+  MLP_CUDA(m, cudaStreamSynchronize(s));
   return ICF_OK;
 }
 
 int icf_mlp_grad_dy(icf_mlp *m, int n, const float *x, const float *dy, float *grad) {
   if (!m || n <= 0 || !x || !dy) return ICF_ERR_ARG;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  if (ensure_cap(m, n)) return ICF_ERR_CUDA;
+  if (ensure_grad(m, n)) return ICF_ERR_CUDA;
   cudaStream_t s = m->stream;
   MLP_CUDA(m, cudaMemcpyAsync(m->d_x, x, sizeof(float) * NI * (size_t)n, cudaMemcpyHostToDevice, s));
-  MLP_CUDA(m, cudaMemcpyAsync(m->d_dy, dy, sizeof(float) * NO * (size_t)n, cudaMemcpyHostToDevice, s));
+  MLP_CUDA(m, cudaMemcpyAsync(m->d_y, dy, sizeof(float) * NO * (size_t)n, cudaMemcpyHostToDevice, s));
   if (grad_on_device(m, n, nullptr, true)) return ICF_ERR_CUDA;
   if (grad) MLP_CUDA(m, cudaMemcpyAsync(grad, m->d_grad, sizeof(float) * NPAR, cudaMemcpyDeviceToHost, s));
   MLP_CUDA(m, cudaStreamSynchronize(s));
@@ -615,7 +730,7 @@ int icf_mlp_train(icf_mlp *m, int n, const float *x, const float *y, int epochs,
   if (!m || n <= 0 || !x || !y || epochs < 1 || batch < 16 || !(lr > 0)) return ICF_ERR_ARG;
   MLP_CUDA(m, cudaSetDevice(m->device));
   if (batch > n) batch = n;
-  if (ensure_cap(m, batch)) return ICF_ERR_CUDA;
+  if (ensure_grad(m, batch)) return ICF_ERR_CUDA;
   cudaStream_t s = m->stream;
   // whole data set on the device, shuffled per epoch on the host (seeded)
   float *dx_all = nullptr, *dy_all = nullptr;
@@ -654,10 +769,10 @@ int icf_mlp_train(icf_mlp *m, int n, const float *x, const float *y, int epochs,
     if (rc == ICF_OK && cudaGetLastError() != cudaSuccess) rc = fail(m, ICF_ERR_CUDA, "training launch failed");
   }
   if (rc == ICF_OK) {
-    // loss over the whole set with the final weights (first `cap` nodes per pass)
+    // loss over the whole set with the final weights (a batch's nodes per pass)
     double tot = 0;
-    for (int b0 = 0; b0 < n && rc == ICF_OK; b0 += m->cap) {
-      const int k = std::min(m->cap, n - b0);
+    for (int b0 = 0; b0 < n && rc == ICF_OK; b0 += batch) {
+      const int k = std::min(batch, n - b0);
       cudaMemcpyAsync(m->d_x, dx_all + (size_t)b0 * NI, sizeof(float) * NI * (size_t)k, cudaMemcpyDeviceToDevice, s);
       cudaMemcpyAsync(m->d_y, dy_all + (size_t)b0 * NO, sizeof(float) * NO * (size_t)k, cudaMemcpyDeviceToDevice, s);
       float l = 0;
