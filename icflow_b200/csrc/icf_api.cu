@@ -205,16 +205,17 @@ int icf_create(int device, icf_ctx **out) {
 
 static void free_all(icf_ctx *c) {
   icf_free_solver(c);
+  icf_free_dyn_ws(c);
   icf_free_tiles(c);
   icf_free_contact_ws(c);
   void *ptrs[] = {c->d_elem, c->d_cz, c->d_alt, c->d_selem, c->d_adj_off, c->d_adj, c->d_faces,
                   c->d_x0, c->d_xc, c->d_va, c->d_u, c->d_v, c->d_a, c->d_du, c->d_un, c->d_h3,
                   c->d_czs, c->d_czfail, c->d_cztent, c->d_czflags, c->d_czavg, c->d_czprm,
                   c->d_es, c->d_cs, c->d_ks, c->d_skeys, c->d_rc_off, c->d_rc, c->d_rows, c->d_cols,
-                  c->d_src, c->d_mkeys, c->d_imp, c->d_cr_slot, c->d_cr_off, c->d_cr, c->d_cr_range, c->d_cr_pslot,
+                  c->d_srow, c->d_mkeys, c->d_imp, c->d_cr_range, c->d_cr_pslot,
                   c->d_cr_row, c->d_pairs,
                   c->d_masks, c->d_rc_mid, c->d_diag, c->d_offd,
-                  c->d_s2m, c->d_dynpos, c->d_gdesc_diag, c->d_vals, c->d_rhs, c->d_nodeF, c->tet_inc.off, c->tet_inc.inc,
+                  c->d_s2m, c->d_gdesc_diag, c->d_vals, c->d_rhs, c->d_nodeF, c->tet_inc.off, c->tet_inc.inc,
                   c->imp_inc.off, c->imp_inc.inc, c->d_tmp, c->sell_off.meta, c->sell_off.unit,
                   c->sell_off.codes, c->sell_diag.meta, c->sell_diag.unit, c->sell_diag.codes,
                   c->sell_off_cz.meta, c->sell_off_cz.unit, c->sell_off_cz.codes, c->sell_diag_cz.meta,
@@ -423,13 +424,13 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
   ctx->d_czavg = nullptr; ctx->d_czprm = nullptr; ctx->d_es = nullptr; ctx->d_cs = nullptr;
   ctx->d_ks = nullptr; ctx->ks_cap = 0;
   ctx->d_rc_mid = ctx->d_diag = ctx->d_offd = nullptr; ctx->n_offd = 0;
-  ctx->d_s2m = ctx->d_dynpos = nullptr; ctx->s2m_cap = ctx->dynpos_cap = ctx->n_dyn = 0;
+  ctx->d_s2m = ctx->d_srow = nullptr; ctx->s2m_cap = 0;
   ctx->d_gdesc_diag = ctx->d_gdesc_off = nullptr; ctx->gdesc_cap = 0; ctx->d_skeys = nullptr; ctx->d_rc_off = nullptr; ctx->d_rc = nullptr;
-  ctx->d_rows = ctx->d_cols = ctx->d_src = nullptr; ctx->rows_cap = ctx->cols_cap = 0; ctx->d_mkeys = nullptr;
-  ctx->d_imp = nullptr; ctx->imp_cap = 0; ctx->n_imp = 0; ctx->d_cr_slot = ctx->d_cr_off = nullptr;
+  ctx->d_rows = ctx->d_cols = nullptr; ctx->rows_cap = ctx->cols_cap = 0; ctx->d_mkeys = nullptr;
+  ctx->d_imp = nullptr; ctx->imp_cap = 0; ctx->n_imp = 0;
   ctx->d_cr_range = nullptr; ctx->d_cr_pslot = ctx->d_cr_row = nullptr;
-  ctx->d_cr = nullptr; ctx->cr_cap = 0; ctx->n_crs = 0; ctx->d_pairs = ctx->d_masks = nullptr;
-  ctx->pairs_cap = 0; ctx->n_pairs = 0; ctx->d_vals = ctx->d_rhs = ctx->d_nodeF = nullptr; ctx->vals_cap = 0;
+  ctx->cr_cap = 0; ctx->n_crs = 0; ctx->d_pairs = ctx->d_masks = nullptr;
+  ctx->pairs_cap = 0; ctx->n_pairs = 0; ctx->d_vals = ctx->d_rhs = ctx->d_nodeF = nullptr; ctx->vals_cap = ctx->rhs_rows = 0;
   ctx->tet_inc = icf_node_inc(); ctx->imp_inc = icf_node_inc(); ctx->d_tmp = nullptr; ctx->tmp_bytes = 0;
   ctx->sell_off = icf_sell();
   ctx->sell_diag = icf_sell();

@@ -42,7 +42,7 @@
 #define ICF_IMP_STAGE 132 // doubles per impact in the staging buffer (allocation)
 // The staging buffer of n impacts holds, from the start, one record of
 // ICF_IMP_REC doubles per impact contribution code, at the code's position in
-// the slot-sorted list d_cr (the 3x3 block of the code's vertex pair, then the
+// the slot-sorted list (the 3x3 block of the code's vertex pair, then the
 // rhs of the vertex on diagonal codes, else zeros; at most 10 codes per
 // impact), and from ICF_IMP_FORCE_AT * n the 12 vertex forces of every impact.
 #define ICF_IMP_REC 12
@@ -168,6 +168,18 @@ struct icf_contact_ws {
   double *h_red = nullptr;  // pinned: the broad phase's grid reduction (7)
 };
 
+// Workspace of the merge of the impacts' blocks into the static pattern
+// (icf_pattern.cu), kept across structures and grown to the high-water mark:
+// per row the codes' count (zero between builds) and offset and the blocks'
+// statistics and their prefix sums; the codes by row; the new columns by row.
+struct icf_dyn_ws {
+  int *cnt = nullptr, *off = nullptr, *newcol = nullptr, *small = nullptr, *h_small = nullptr;
+  int4 *stat = nullptr, *pre = nullptr;
+  unsigned long long *items = nullptr;
+  long long items_cap = 0;
+  int rows_cap = 0;
+};
+
 // Device MINRES solver state (icf_solve.cu).
 struct icf_solver {
   // row order (position -> row and back), of order_rows rows
@@ -287,10 +299,11 @@ struct icf_ctx {
   // diagonal slot per row (-1 if none), compacted off-diagonal slots
   int *d_rc_mid = nullptr, *d_diag = nullptr, *d_offd = nullptr;
   int n_offd = 0;
-  // static -> merged slot (when contact pairs add blocks) and the merged
-  // positions of the contact-only blocks
-  int *d_s2m = nullptr, *d_dynpos = nullptr;
-  int s2m_cap = 0, dynpos_cap = 0, n_dyn = 0;
+  // static -> merged slot (when contact pairs add blocks), the static rows'
+  // first slots, and the workspace of the merge
+  int *d_s2m = nullptr, *d_srow = nullptr;
+  int s2m_cap = 0;
+  icf_dyn_ws dyn;
   // gather descriptors {merged position, first tet code, first CZ code, end}:
   // N per-row diagonal entries, then one per off-diagonal block (one buffer)
   int4 *d_gdesc_diag = nullptr, *d_gdesc_off = nullptr;
@@ -317,7 +330,7 @@ struct icf_ctx {
   bool lists_static = false;
 
   // merged pattern
-  int *d_rows = nullptr, *d_cols = nullptr, *d_src = nullptr;
+  int *d_rows = nullptr, *d_cols = nullptr;
   int rows_cap = 0, cols_cap = 0;
   unsigned long long *d_mkeys = nullptr;
 
@@ -339,17 +352,16 @@ struct icf_ctx {
   // per-impact classification {kind, ia, ib, 0} and {s, t, dsq, 0}; same
   // capacity as the impact staging d_ks (ks_cap)
   int n_crs = 0;                  // slots touched by impacts
-  int *d_cr_slot = nullptr, *d_cr_off = nullptr;
-  uint32_t *d_cr = nullptr;
   int cr_cap = 0;
   // the touched slots in k_imp_add's order: those the off-diagonal gather
   // does not write (diagonal and contact-only blocks, n_crs - n_crs_off)
   // first, then the static off-diagonal ones, so that each k_imp_add launch
-  // covers its own contiguous range: per slot its records' range in d_cr,
-  // the slot and, for a diagonal block, its rhs row (else -1)
+  // covers its own contiguous range: per slot the range of its codes in the
+  // slot-sorted list of the impacts' codes, the slot and, for a diagonal
+  // block, its rhs row (else -1, or -2 for a contact-only block)
   int2 *d_cr_range = nullptr;
   int *d_cr_pslot = nullptr, *d_cr_row = nullptr;
-  // position in d_cr of the code (impact u, vertices a, b) at 16 u + 4 a + b,
+  // position in that list of the code (impact u, vertices a, b) at 16 u + 4 a + b,
   // or -1 (no code: an anchored vertex, or the pair taken as (b, a))
   int *d_imp_pos = nullptr;
   long long imp_pos_cap = 0;
@@ -371,7 +383,7 @@ struct icf_ctx {
 
   // outputs
   double *d_vals = nullptr, *d_rhs = nullptr, *d_nodeF = nullptr;
-  int vals_cap = 0;
+  int vals_cap = 0, rhs_rows = 0;
 
   // counters: [0] damaged [1] failed [2] contact [3] active impacts [4] nonfinite
   // [5] undecided CZ law comparisons
@@ -449,11 +461,6 @@ int icf_launch_tile_fused(icf_ctx *ctx, const double4 *xc, const double2 *va, co
 inline bool icf_fused_active(const icf_ctx *ctx) { return ctx->fused_tiles && icf_tiles_active(ctx); }
 int icf_rebuild_lists(icf_ctx *ctx);  // both gathers' lists for the current layout and split
 int icf_remap_lists(icf_ctx *ctx);    // their units' slots for the current structure
-// 1 for a merged slot that the off-diagonal gather writes: static, off the diagonal
-__host__ __device__ inline bool icf_off_static(const unsigned long long *mkey, const int *src, int identity, int s) {
-  const unsigned long long k = mkey[s];
-  return (identity || src[s] >= 0) && (k >> 32) != (k & 0xffffffffull);
-}  // both gathers' lists for the current layout and split
 int icf_rebuild_sell_diag(icf_ctx *ctx, int lanes);
 int icf_rebuild_sell_off(icf_ctx *ctx, bool natural);
 // position map and zeroed contribution staging for the current lists
@@ -467,6 +474,7 @@ int icf_launch_law_eval(icf_ctx *ctx, int n, const double *in, const double4 *pr
 int icf_settle_law(icf_ctx *ctx, const std::function<int()> &rerun);
 int icf_solve_impl(icf_ctx *ctx, double rel_tol, int max_iter, int *iters, double *relres);
 void icf_free_solver(icf_ctx *ctx);
+void icf_free_dyn_ws(icf_ctx *ctx);
 int icf_launch_sumsq(icf_ctx *ctx, const double *d_x, long long n);
 int icf_broad_phase_impl(icf_ctx *ctx, double pad, const int *d_group, int *n_pairs_out);
 void icf_free_contact_ws(icf_ctx *ctx);

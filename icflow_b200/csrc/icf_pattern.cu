@@ -13,6 +13,14 @@
 // paired with a 32-bit contribution code.  A stable radix sort by key puts
 // the contributions of every block next to each other, in unit order; the
 // run heads are the slots.  That sorted code list is what k_gather walks.
+//
+// The dynamic part changes with every contact list, so it avoids sorting it
+// as a whole: the impacts' blocks are counted and placed by row, and one warp
+// per row sorts the few of its row and merges them with the row's static
+// blocks.  (A 64-bit radix sort of 16 keys per impact, another of the codes by
+// slot, run-length encodings and six synchronisations took 410 us of kernels
+// and as much again of allocations and waiting at 22,687 impacts, 490 us a call;
+// this takes 100 us of kernels and 138 us a call, one synchronisation among it.)
 #include <cub/cub.cuh>
 
 #include "icf_internal.cuh"
@@ -99,60 +107,256 @@ __global__ void k_cols(int nnz, const unsigned long long *__restrict__ key, int 
   cols[s] = (int)(key[s] & 0xffffffffull);
 }
 
-__global__ void k_cand_dyn(int ni, const int4 *__restrict__ imp, const int *__restrict__ alt,
-                           unsigned long long *__restrict__ key) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= ni) return;
-  const int4 id = imp[u];
+// ---- the impacts' blocks ----------------------------------------------------------
+// A code (impact u, vertices a, b), u << 4 | a << 2 | b, belongs to row alt(a) when
+// both vertices are active and alt(b) >= alt(a); on the diagonal only where
+// the static pattern has the row's diagonal block (contact adds none).
+// bad: a block off the diagonal in a row outside the pattern.
+template <class F>
+__device__ __forceinline__ void imp_codes(int u, const int4 id, const int *__restrict__ alt, int N,
+                                          const int *__restrict__ diag, int *__restrict__ bad, F f) {
   const int nid[4] = {id.x, id.y, id.z, id.w};
   int al[4];
-  for (int i = 0; i < 4; i++) al[i] = nid[i] >= 0 ? alt[nid[i]] : -1;
+#pragma unroll
+  for (int i = 0; i < 4; i++) al[i] = nid[i] >= 0 ? __ldg(alt + nid[i]) : -1;
+#pragma unroll
   for (int a = 0; a < 4; a++)
+#pragma unroll
     for (int b = 0; b < 4; b++) {
-      const bool ok = al[a] >= 0 && al[b] >= 0 && al[b] > al[a];
-      key[16 * (size_t)u + 4 * a + b] = ok ? (((unsigned long long)al[a] << 32) | (unsigned)al[b]) : KMAX;
+      if (al[a] < 0 || al[b] < al[a]) continue;
+      if (al[a] >= N) {
+        if (al[b] > al[a]) atomicOr(bad, 1);
+        continue;
+      }
+      if (al[b] == al[a] && __ldg(diag + al[a]) < 0) continue;
+      f(al[a], al[b], (unsigned)u << 4 | (unsigned)(a << 2 | b));
     }
 }
 
-// keep dynamic keys that are new (not in the static pattern); flag rows that
-// fall outside the pattern (the reference would throw there)
-__global__ void k_dyn_new(int n, const unsigned long long *__restrict__ dkey,
-                          const unsigned long long *__restrict__ skey, int nnz_s, int N,
-                          int *__restrict__ keep, int *__restrict__ bad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned long long k = dkey[i];
-  int kp = 0;
-  if (k != KMAX) {
-    if ((int)(k >> 32) >= N) atomicOr(bad, 1);
-    const long long p = lower_bound_u64(skey, nnz_s, k);
-    kp = !(p < nnz_s && skey[p] == k);
-  }
-  keep[i] = kp;
+// codes per row; pos (16 per impact) preset to "no code"
+__global__ void k_imp_count(int ni, const int4 *__restrict__ imp, const int *__restrict__ alt, int N,
+                            const int *__restrict__ diag, int *__restrict__ cnt, int4 *__restrict__ pos,
+                            int *__restrict__ bad) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= ni) return;
+#pragma unroll
+  for (int k = 0; k < 4; k++) pos[4 * (size_t)u + k] = make_int4(-1, -1, -1, -1);
+  imp_codes(u, imp[u], alt, N, diag, bad, [&](int row, int, unsigned) { atomicAdd(cnt + row, 1); });
 }
 
-__global__ void k_merge_static(int nnz_s, const unsigned long long *__restrict__ skey,
-                               const unsigned long long *__restrict__ dkey, int nd,
-                               unsigned long long *__restrict__ mkey, int *__restrict__ src,
-                               int *__restrict__ s2m) {
+// the codes by row, items {column, code}, in any order; cnt counts down to zero
+__global__ void k_imp_place(int ni, const int4 *__restrict__ imp, const int *__restrict__ alt, int N,
+                            const int *__restrict__ diag, const int *__restrict__ off, int *__restrict__ cnt,
+                            unsigned long long *__restrict__ items, int *__restrict__ bad) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= ni) return;
+  imp_codes(u, imp[u], alt, N, diag, bad, [&](int row, int col, unsigned code) {
+    items[off[row] + atomicSub(cnt + row, 1) - 1] = (unsigned long long)(unsigned)col << 32 | code;
+  });
+}
+
+// index of the first of n ascending keys that is >= key
+__device__ __forceinline__ int lower_of(const unsigned long long *__restrict__ k, int n, unsigned long long key) {
+  int lo = 0;
+  while (lo < n) {
+    const int mid = (lo + n) >> 1;
+    if (k[mid] < key) lo = mid + 1;
+    else n = mid;
+  }
+  return lo;
+}
+
+// The static blocks of a row for a warp's searches: up to 32 columns in its
+// lanes (compared with by shuffles: the loads of a binary search would wait
+// for one another), more by binary search.
+struct row_cols {
+  const unsigned long long *key;
+  int n;
+  unsigned c;  // lane's column
+  __device__ __forceinline__ row_cols(const unsigned long long *skey, int s0, int s1, int lane) {
+    key = skey + s0;
+    n = s1 - s0;
+    c = lane < n ? (unsigned)key[lane] : 0xffffffffu;
+  }
+  // columns below col, and whether col is one of them (all lanes take part)
+  __device__ __forceinline__ int find(int r, unsigned col, bool &found) const {
+    int p = 0;
+    found = false;
+    if (n <= 32) {
+      for (int t = 0; t < n; t++) {
+        const unsigned x = __shfl_sync(0xffffffffu, c, t);
+        p += x < col;
+        found |= x == col;
+      }
+      return p;
+    }
+    const unsigned long long k = (unsigned long long)(unsigned)r << 32 | col;
+    p = lower_of(key, n, k);
+    found = p < n && key[p] == k;
+    return p;
+  }
+};
+
+struct int4_sum {
+  __host__ __device__ int4 operator()(const int4 &a, const int4 &b) const {
+    return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+  }
+};
+
+// One warp per row: its items in ascending order (columns, then codes: unit
+// order) and, for the scan, its blocks: {new, touched diagonal or new, touched
+// static off the diagonal, 0}.  Up to 32 items sort in registers, more by a
+// bitonic network in place whose missing items count as infinite (all its
+// comparisons point one way, so it needs no padding).  Bound by the chain row ->
+// offset -> items and columns (20 us at 22,687 impacts, which touch 19,000 of
+// 56,603 rows; a list of the touched rows took 17 us and 10 us to make, eight
+// rows one after the other in a warp 24 us).
+__global__ void __launch_bounds__(256) k_imp_sort(int N, const int *__restrict__ off,
+                                                  unsigned long long *__restrict__ items,
+                                                  const int *__restrict__ srow,
+                                                  const unsigned long long *__restrict__ skey,
+                                                  int4 *__restrict__ stat) {
+  const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (r > N) return;
+  const int b = r < N ? off[r] : 0, n = r < N ? off[r + 1] - b : 0;
+  const int s0 = r < N ? srow[r] : 0, s1 = r < N ? srow[r + 1] : 0;
+  if (n == 0) {
+    if (lane == 0) stat[r] = make_int4(0, 0, 0, 0);
+    return;
+  }
+  unsigned long long *it = items + b;
+  const row_cols C(skey, s0, s1, lane);
+  unsigned long long v = KMAX;
+  if (n <= 32) {
+    if (lane < n) v = it[lane];
+    for (int k = 2; k < 2 * n; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const int m = j == k >> 1 ? k - 1 : j;  // first against the mirror image
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, m);
+        v = lane < (lane ^ m) ? (o < v ? o : v) : (o > v ? o : v);
+      }
+    if (lane < n) it[lane] = v;
+  } else {
+    for (int k = 2; k < 2 * n; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+          const int m = j == k >> 1 ? (i ^ (k - 1)) : (i ^ j);
+          if (m > i && m < n) {
+            const unsigned long long x = it[i], y = it[m];
+            if (y < x) {
+              it[i] = y;
+              it[m] = x;
+            }
+          }
+        }
+      }
+    __syncwarp();
+  }
+  int na = 0, no = 0, nn = 0;
+  unsigned last = 0xffffffffu;  // column of the item before this round's
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    if (n > 32) v = i0 + lane < n ? it[i0 + lane] : KMAX;
+    const unsigned col = (unsigned)(v >> 32);
+    unsigned prev = __shfl_up_sync(0xffffffffu, col, 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(0xffffffffu, col, 31);
+    bool found;
+    C.find(r, col, found);
+    const bool head = i0 + lane < n && (i0 + lane == 0 || prev != col), diag = col == (unsigned)r;
+    nn += head && !found;
+    na += head && (!found || diag);
+    no += head && found && !diag;
+  }
+  na = __reduce_add_sync(0xffffffffu, na);
+  no = __reduce_add_sync(0xffffffffu, no);
+  nn = __reduce_add_sync(0xffffffffu, nn);
+  if (lane == 0) stat[r] = make_int4(nn, na, no, 0);
+}
+
+// One warp per row: the merged row start; the new blocks (merged position,
+// key, column; their columns row by row in newcol); every code's place; the
+// touched blocks in k_imp_add's order, a stable partition: diagonal and
+// contact-only blocks at [0, n_a), static off-diagonal ones from n_a, each part
+// in slot order (so a warp's records and blocks lie close together): record
+// range, slot and rhs row (diagonal blocks), -1 (static off-diagonal blocks) or
+// -2 (contact-only blocks, which k_imp_add writes rather than adds to).
+__global__ void __launch_bounds__(256) k_imp_write(int N, int n_a, const int *__restrict__ off,
+                                                   const unsigned long long *__restrict__ items,
+                                                   const int *__restrict__ srow,
+                                                   const unsigned long long *__restrict__ skey,
+                                                   const int4 *__restrict__ pre, int *__restrict__ rows,
+                                                   unsigned long long *__restrict__ mkey, int *__restrict__ cols,
+                                                   int *__restrict__ newcol, int *__restrict__ pos,
+                                                   int2 *__restrict__ range, int *__restrict__ pslot,
+                                                   int *__restrict__ prow) {
+  const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (r > N) return;
+  const int4 o = pre[r];
+  const int s0 = srow[r], b = r < N ? off[r] : 0, n = r < N ? off[r + 1] - b : 0, s1 = r < N ? srow[r + 1] : s0;
+  if (lane == 0) rows[r] = s0 + o.x;
+  if (n == 0) return;
+  const unsigned long long *it = items + b;
+  const row_cols C(skey, s0, s1, lane);
+  int nn = 0, na = 0, no = 0;  // blocks of the row before this round's
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const int i = i0 + lane;
+    const unsigned long long v = i < n ? it[i] : KMAX;
+    const unsigned col = (unsigned)(v >> 32);
+    unsigned prev = __shfl_up_sync(0xffffffffu, col, 1);
+    if (lane == 0 && i0 > 0) prev = (unsigned)(it[i0 - 1] >> 32);
+    if (i < n) pos[(unsigned)v] = b + i;
+    bool found;
+    const int p = C.find(r, col, found);
+    const bool head = i < n && (i == 0 || prev != col), is_new = !found, diag = col == (unsigned)r;
+    const unsigned below = (1u << lane) - 1;
+    const unsigned mn = __ballot_sync(0xffffffffu, head && is_new);
+    const unsigned ma = __ballot_sync(0xffffffffu, head && (is_new || diag));
+    const unsigned mo = __ballot_sync(0xffffffffu, head && !is_new && !diag);
+    if (head) {
+      const int j = nn + __popc(mn & below);
+      const int slot = s0 + p + o.x + j;
+      // the run ends at the next head, or beyond this round
+      const unsigned after = (ma | mo) & ~below & ~(1u << lane);
+      int e = after ? i0 + __ffs(after) - 1 : min(n, i0 + 32);
+      if (!after)
+        while (e < n && (unsigned)(it[e] >> 32) == col) e++;
+      const int w = is_new || diag ? o.y + na + __popc(ma & below) : n_a + o.z + no + __popc(mo & below);
+      range[w] = make_int2(b + i, b + e);
+      pslot[w] = slot;
+      prow[w] = diag ? r : (is_new ? -2 : -1);
+      if (is_new) {
+        newcol[o.x + j] = (int)col;
+        mkey[slot] = (unsigned long long)(unsigned)r << 32 | col;
+        cols[slot] = (int)col;
+      }
+    }
+    nn += __popc(mn);
+    na += __popc(ma);
+    no += __popc(mo);
+  }
+}
+
+// the static blocks' merged positions: behind the new blocks of the rows
+// before and those of their row with smaller columns
+__global__ void k_merge_static(int nnz_s, const unsigned long long *__restrict__ skey, const int4 *__restrict__ pre,
+                               const int *__restrict__ newcol, unsigned long long *__restrict__ mkey,
+                               int *__restrict__ cols, int *__restrict__ s2m) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nnz_s) return;
-  const long long p = i + lower_bound_u64(dkey, nd, skey[i]);
-  mkey[p] = skey[i];
-  src[p] = i;
-  s2m[i] = (int)p;
-}
-
-__global__ void k_merge_dyn(int nd, const unsigned long long *__restrict__ dkey,
-                            const unsigned long long *__restrict__ skey, int nnz_s,
-                            unsigned long long *__restrict__ mkey, int *__restrict__ src,
-                            int *__restrict__ dynpos) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nd) return;
-  const long long p = j + lower_bound_u64(skey, nnz_s, dkey[j]);
-  mkey[p] = dkey[j];
-  src[p] = -1;
-  dynpos[j] = (int)p;
+  const unsigned long long k = skey[i];
+  const int r = (int)(k >> 32), c = (int)(k & 0xffffffffull);
+  const int o = __ldg(&pre[r].x), e = __ldg(&pre[r + 1].x);
+  int lo = o, hi = e;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (newcol[mid] < c) lo = mid + 1;
+    else hi = mid;
+  }
+  const int p = i + lo;
+  mkey[p] = k;
+  cols[p] = c;
+  s2m[i] = p;
 }
 
 // Per static slot: where its CZ codes start (tet codes come first in the
@@ -273,69 +477,6 @@ __global__ void k_off_codes(int n, const int *__restrict__ offflag, const int *_
 __global__ void k_iota(int n, int *__restrict__ a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = i;
-}
-
-// impact contributions keyed by their merged slot
-// 1 where the touched slot is a static off-diagonal block (written by the
-// off-diagonal gather), else 0; flag[n] = 0
-__global__ void k_flag_off(int n, const int *__restrict__ slot, const unsigned long long *__restrict__ mkey,
-                           const int *__restrict__ src, int identity, int *__restrict__ flag) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > n) return;
-  flag[g] = g < n && icf_off_static(mkey, src, identity, slot[g]) ? 1 : 0;
-}
-
-// the touched slots in k_imp_add's order, a stable partition: diagonal and
-// contact-only blocks at [0, n_a), static off-diagonal ones at [n_a, n), each
-// part in slot order (so a warp's records and blocks lie close together); per
-// slot its record range, slot and rhs row (diagonal blocks), -1 (static
-// off-diagonal blocks) or -2 (contact-only blocks, which k_imp_add writes
-// rather than adds to).  pref: the exclusive prefix sum of k_flag_off's flags.
-__global__ void k_split_off(int n, int n_a, const int *__restrict__ slot, const int *__restrict__ off,
-                            const unsigned long long *__restrict__ mkey, const int *__restrict__ pref,
-                            int2 *__restrict__ range, int *__restrict__ pslot, int *__restrict__ row) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n) return;
-  const int sl = slot[g];
-  const bool f = pref[g + 1] != pref[g];
-  const int p = f ? n_a + pref[g] : g - pref[g];
-  range[p] = make_int2(off[g], off[g + 1]);
-  pslot[p] = sl;
-  const unsigned long long k = mkey[sl];
-  row[p] = (k >> 32) == (k & 0xffffffffull) ? (int)(k & 0xffffffffull) : (f ? -1 : -2);
-}
-
-__global__ void k_cand_imp_rc(int ni, const int4 *__restrict__ imp, const int *__restrict__ alt,
-                              const unsigned long long *__restrict__ mkey, int nnz,
-                              int *__restrict__ slot, uint32_t *__restrict__ code) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= ni) return;
-  const int4 id = imp[u];
-  const int nid[4] = {id.x, id.y, id.z, id.w};
-  int al[4];
-  for (int i = 0; i < 4; i++) al[i] = nid[i] >= 0 ? alt[nid[i]] : -1;
-  for (int a = 0; a < 4; a++)
-    for (int b = 0; b < 4; b++) {
-      const size_t o = 16 * (size_t)u + 4 * a + b;
-      int s = 0x7fffffff;
-      if (al[a] >= 0 && al[b] >= 0 && al[b] >= al[a]) {
-        const unsigned long long k = ((unsigned long long)al[a] << 32) | (unsigned)al[b];
-        const long long p = lower_bound_u64(mkey, nnz, k);
-        if (p < nnz && mkey[p] == k) s = (int)p;
-      }
-      slot[o] = s;
-      code[o] = icf_code_tet(ICF_KIND_IMP, u, a, b);
-    }
-}
-
-// pos[16 u + 4 a + b] = position of impact code (u, a, b) in the slot-sorted
-// list, for the valid codes (those before the invalid-slot run)
-__global__ void k_imp_pos(int n, const int *__restrict__ n_valid, const uint32_t *__restrict__ code,
-                          int *__restrict__ pos) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n || q >= *n_valid) return;
-  const uint32_t c = code[q];
-  pos[16 * (size_t)((c >> 4) & 0x3FFFFFFu) + (c & 15u)] = q;
 }
 
 // node incidence lists: (node, unit << 2 | vertex)
@@ -475,6 +616,8 @@ int icf_build_static_pattern(icf_ctx *ctx) {
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_skeys, sizeof(unsigned long long)));
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_rc_off, sizeof(int)));
     ICF_CUDA(ctx, cudaMemset(ctx->d_rc_off, 0, sizeof(int)));
+    ICF_CUDA(ctx, cudaMalloc(&ctx->d_srow, sizeof(int)));
+    ICF_CUDA(ctx, cudaMemset(ctx->d_srow, 0, sizeof(int)));
     return ICF_OK;
   }
   unsigned long long *k0, *k1;
@@ -539,8 +682,12 @@ int icf_build_static_pattern(icf_ctx *ctx) {
   ctx->N = nnz_s > 0 ? (int)(last >> 32) + 1 : 0;
 
   // gather metadata: CZ-code start per slot, diagonal slot per row, the
-  // compacted list of off-diagonal slots
+  // compacted list of off-diagonal slots; the rows' first slots
   const int N = ctx->N;
+  cudaFree(ctx->d_srow);
+  ctx->d_srow = nullptr;
+  ICF_CUDA(ctx, cudaMalloc(&ctx->d_srow, sizeof(int) * (size_t)(N + 1)));
+  k_rows<<<icf_blocks((long long)N + 1, 256), 256, 0, s>>>(N, nnz_s, ctx->d_skeys, ctx->d_srow);
   cudaFree(ctx->d_rc_mid);
   cudaFree(ctx->d_diag);
   cudaFree(ctx->d_offd);
@@ -737,99 +884,116 @@ static int build_lists(icf_ctx *ctx, bool off, bool diag) {
 }
 
 template <typename T>
-static int grow(icf_ctx *ctx, T **p, int *cap, long long n) {
-  if (n <= *cap && *p) return ICF_OK;
+static int grow(icf_ctx *ctx, T **p, long long n) {
   cudaFree(*p);
   *p = nullptr;
-  const long long c = n + n / 4 + 16;
-  ICF_CUDA(ctx, cudaMalloc(p, sizeof(T) * (size_t)c));
-  *cap = (int)c;
+  ICF_CUDA(ctx, cudaMalloc(p, sizeof(T) * (size_t)n));
   return ICF_OK;
+}
+
+void icf_free_dyn_ws(icf_ctx *ctx) {
+  icf_dyn_ws &D = ctx->dyn;
+  void *ptrs[] = {D.cnt, D.off, D.stat, D.pre, D.items, D.newcol, D.small};
+  for (void *p : ptrs) cudaFree(p);
+  cudaFreeHost(D.h_small);
+  D = icf_dyn_ws();
 }
 
 int icf_build_merged_pattern(icf_ctx *ctx) {
   cudaStream_t s = ctx->stream;
-  const int nnz_s = ctx->nnz_s, N = ctx->N;
-  int nd = 0;
-  unsigned long long *dkeys = nullptr;
-  if (ctx->n_imp > 0) {
-    const int n = 16 * ctx->n_imp;
-    unsigned long long *a, *b;
-    int *keep, *d_nd, *d_bad;
-    ICF_CUDA(ctx, cudaMallocAsync(&a, sizeof(unsigned long long) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&b, sizeof(unsigned long long) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&keep, sizeof(int) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&d_nd, sizeof(int) * 2, s));
-    d_bad = d_nd + 1;
-    ICF_CUDA(ctx, cudaMemsetAsync(d_nd, 0, sizeof(int) * 2, s));
-    k_cand_dyn<<<icf_blocks(ctx->n_imp, 128), 128, 0, s>>>(ctx->n_imp, ctx->d_imp, ctx->d_alt, a);
-    size_t tb = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, tb, a, b, n, 0, 64, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceRadixSort::SortKeys(ctx->d_tmp, tb, a, b, n, 0, 64, s));
-    tb = 0;
-    cub::DeviceSelect::Unique(nullptr, tb, b, a, d_nd, n, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceSelect::Unique(ctx->d_tmp, tb, b, a, d_nd, n, s));
-    int nu = 0;
-    ICF_CUDA(ctx, cudaMemcpyAsync(&nu, d_nd, sizeof(int), cudaMemcpyDeviceToHost, s));
+  const int nnz_s = ctx->nnz_s, N = ctx->N, ni = ctx->n_imp;
+  icf_dyn_ws &D = ctx->dyn;
+  int4 tot = make_int4(0, 0, 0, 0);  // new blocks; touched ones of each part
+  if (ni > 0) {
+    // per-row work arrays (cnt stays zero between builds) and the items
+    if (N + 1 > D.rows_cap) {
+      const long long c = N + 1LL;
+      ICF_TRY_RC(grow(ctx, &D.cnt, c));
+      ICF_TRY_RC(grow(ctx, &D.off, c));
+      ICF_TRY_RC(grow(ctx, &D.stat, c));
+      ICF_TRY_RC(grow(ctx, &D.pre, c));
+      ICF_CUDA(ctx, cudaMemsetAsync(D.cnt, 0, sizeof(int) * (size_t)c, s));
+      if (!D.small) ICF_CUDA(ctx, cudaMalloc(&D.small, sizeof(int)));
+      if (!D.h_small) ICF_CUDA(ctx, cudaMallocHost(&D.h_small, 8 * sizeof(int)));
+      D.rows_cap = N + 1;
+    }
+    if (16LL * ni > D.items_cap) {
+      const long long c = 16LL * ni + 4LL * ni;
+      ICF_TRY_RC(grow(ctx, &D.items, c));
+      ICF_TRY_RC(grow(ctx, &D.newcol, c));
+      D.items_cap = c;
+    }
+    if (16LL * ni > ctx->imp_pos_cap || !ctx->d_imp_pos) {
+      ICF_TRY_RC(grow(ctx, &ctx->d_imp_pos, 32LL * ni));
+      ctx->imp_pos_cap = 32LL * ni;
+    }
+    size_t tb = 0, tb2 = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, D.cnt, D.off, N + 1, s);
+    cub::DeviceScan::ExclusiveScan(nullptr, tb2, D.stat, D.pre, int4_sum(), make_int4(0, 0, 0, 0), N + 1, s);
+    if (icf_scratch(ctx, tb > tb2 ? tb : tb2)) return ICF_ERR_CUDA;
+    ICF_CUDA(ctx, cudaMemsetAsync(D.small, 0, sizeof(int), s));
+    k_imp_count<<<icf_blocks(ni, 128), 128, 0, s>>>(ni, ctx->d_imp, ctx->d_alt, N, ctx->d_diag, D.cnt,
+                                                   reinterpret_cast<int4 *>(ctx->d_imp_pos), D.small);
+    ICF_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->d_tmp, tb, D.cnt, D.off, N + 1, s));
+    k_imp_place<<<icf_blocks(ni, 128), 128, 0, s>>>(ni, ctx->d_imp, ctx->d_alt, N, ctx->d_diag, D.off, D.cnt, D.items,
+                                                   D.small);
+    k_imp_sort<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, D.off, D.items, ctx->d_srow, ctx->d_skeys, D.stat);
+    ICF_CUDA(ctx, cub::DeviceScan::ExclusiveScan(ctx->d_tmp, tb2, D.stat, D.pre, int4_sum(), make_int4(0, 0, 0, 0),
+                                                 N + 1, s));
+    ICF_CUDA(ctx, cudaGetLastError());
+    ICF_CUDA(ctx, cudaMemcpyAsync(D.h_small, D.pre + N, sizeof(int4), cudaMemcpyDeviceToHost, s));
+    ICF_CUDA(ctx, cudaMemcpyAsync(D.h_small + 4, D.small, sizeof(int), cudaMemcpyDeviceToHost, s));
     ICF_CUDA(ctx, cudaStreamSynchronize(s));
-    if (nu > 0) k_dyn_new<<<icf_blocks(nu, 128), 128, 0, s>>>(nu, a, ctx->d_skeys, nnz_s, N, keep, d_bad);
-    tb = 0;
-    cub::DeviceSelect::Flagged(nullptr, tb, a, keep, b, d_nd, nu, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceSelect::Flagged(ctx->d_tmp, tb, a, keep, b, d_nd, nu, s));
-    int hb[2] = {0, 0};
-    ICF_CUDA(ctx, cudaMemcpyAsync(hb, d_nd, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));
-    ICF_CUDA(ctx, cudaStreamSynchronize(s));
-    nd = hb[0];
-    if (hb[1]) return icf_fail(ctx, ICF_ERR_STATE, "an impact references a row outside the pattern");
-    dkeys = b;
-    ICF_CUDA(ctx, cudaFreeAsync(a, s));
-    ICF_CUDA(ctx, cudaFreeAsync(keep, s));
-    ICF_CUDA(ctx, cudaFreeAsync(d_nd, s));
+    if (D.h_small[4]) return icf_fail(ctx, ICF_ERR_STATE, "an impact references a row outside the pattern");
+    tot = make_int4(D.h_small[0], D.h_small[1], D.h_small[2], 0);
   }
-  const int nnz = nnz_s + nd;
+  const int nd = tot.x, nnz = nnz_s + nd;
   if (nnz + 1 > ctx->cols_cap || !ctx->d_cols) {
-    cudaFree(ctx->d_cols);
-    cudaFree(ctx->d_src);
-    cudaFree(ctx->d_mkeys);
-    ctx->d_cols = ctx->d_src = nullptr;
-    ctx->d_mkeys = nullptr;
     const long long cap = nnz + 1 + nnz / 8 + 64;
-    ICF_CUDA(ctx, cudaMalloc(&ctx->d_cols, sizeof(int) * (size_t)cap));
-    ICF_CUDA(ctx, cudaMalloc(&ctx->d_src, sizeof(int) * (size_t)cap));
-    ICF_CUDA(ctx, cudaMalloc(&ctx->d_mkeys, sizeof(unsigned long long) * (size_t)cap));
+    ICF_TRY_RC(grow(ctx, &ctx->d_cols, cap));
+    ICF_TRY_RC(grow(ctx, &ctx->d_mkeys, cap));
     ctx->cols_cap = (int)cap;
   }
-  int rc = grow(ctx, &ctx->d_rows, &ctx->rows_cap, (long long)N + 1);
-  if (rc) return rc;
-  if (nd == 0) {
+  if (N + 1 > ctx->rows_cap || !ctx->d_rows) {
+    ICF_TRY_RC(grow(ctx, &ctx->d_rows, N + 1LL));
+    ctx->rows_cap = N + 1;
+  }
+  if (ni == 0) {
     ICF_CUDA(ctx, cudaMemcpyAsync(ctx->d_mkeys, ctx->d_skeys, sizeof(unsigned long long) * (size_t)nnz_s,
                                   cudaMemcpyDeviceToDevice, s));
-    ctx->src_identity = true;
+    if (nnz > 0) k_cols<<<icf_blocks(nnz, 256), 256, 0, s>>>(nnz, ctx->d_mkeys, ctx->d_cols);
+    k_rows<<<icf_blocks((long long)N + 1, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, ctx->d_rows);
   } else {
-    // static -> merged positions and the positions of the contact-only blocks
     if (!ctx->d_s2m || ctx->s2m_cap < nnz_s + 1) {
-      cudaFree(ctx->d_s2m);
-      ctx->d_s2m = nullptr;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_s2m, sizeof(int) * (size_t)(nnz_s + 1)));
+      ICF_TRY_RC(grow(ctx, &ctx->d_s2m, nnz_s + 1LL));
       ctx->s2m_cap = nnz_s + 1;
     }
-    if (!ctx->d_dynpos || ctx->dynpos_cap < nd) {
-      cudaFree(ctx->d_dynpos);
-      ctx->d_dynpos = nullptr;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_dynpos, sizeof(int) * (size_t)(2 * nd)));
-      ctx->dynpos_cap = 2 * nd;
+    const int n_crs = tot.y + tot.z;
+    if (n_crs > ctx->cr_cap || !ctx->d_cr_range) {
+      const long long c = n_crs + n_crs / 4 + 16;
+      ICF_TRY_RC(grow(ctx, &ctx->d_cr_range, c));
+      ICF_TRY_RC(grow(ctx, &ctx->d_cr_pslot, c));
+      ICF_TRY_RC(grow(ctx, &ctx->d_cr_row, c));
+      ctx->cr_cap = (int)c;
     }
+    k_imp_write<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, tot.y, D.off, D.items, ctx->d_srow, ctx->d_skeys,
+                                                              D.pre, ctx->d_rows, ctx->d_mkeys, ctx->d_cols, D.newcol,
+                                                              ctx->d_imp_pos, ctx->d_cr_range, ctx->d_cr_pslot,
+                                                              ctx->d_cr_row);
     if (nnz_s > 0)
-      k_merge_static<<<icf_blocks(nnz_s, 256), 256, 0, s>>>(nnz_s, ctx->d_skeys, dkeys, nd, ctx->d_mkeys,
-                                                           ctx->d_src, ctx->d_s2m);
-    k_merge_dyn<<<icf_blocks(nd, 256), 256, 0, s>>>(nd, dkeys, ctx->d_skeys, nnz_s, ctx->d_mkeys, ctx->d_src,
-                                                   ctx->d_dynpos);
-    ctx->src_identity = false;
+      k_merge_static<<<icf_blocks(nnz_s, 256), 256, 0, s>>>(nnz_s, ctx->d_skeys, D.pre, D.newcol, ctx->d_mkeys,
+                                                           ctx->d_cols, ctx->d_s2m);
+    // impact staging
+    if (ni > ctx->ks_cap) {
+      ICF_TRY_RC(grow(ctx, &ctx->d_ks, (long long)ICF_IMP_STAGE * 2 * ni));
+      ctx->ks_cap = 2 * ni;
+    }
   }
-  ctx->n_dyn = nd;
+  ICF_CUDA(ctx, cudaGetLastError());
+  ctx->src_identity = nd == 0;
+  ctx->nnz = nnz;
+  ctx->n_crs = tot.y + tot.z;
+  ctx->n_crs_off = tot.z;
   // gather descriptors for this merge
   if (!ctx->d_gdesc_diag || ctx->gdesc_cap < N + ctx->n_offd + 2) {
     cudaFree(ctx->d_gdesc_diag);
@@ -856,115 +1020,6 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
   }
   if (icf_remap_lists(ctx)) return ICF_ERR_CUDA;
   if (ctx->tiles.built && icf_remap_tiles(ctx)) return ICF_ERR_CUDA;
-  if (dkeys) ICF_CUDA(ctx, cudaFreeAsync(dkeys, s));
-  if (nnz > 0) k_cols<<<icf_blocks(nnz, 256), 256, 0, s>>>(nnz, ctx->d_mkeys, ctx->d_cols);
-  k_rows<<<icf_blocks((long long)N + 1, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, ctx->d_rows);
-  ICF_CUDA(ctx, cudaGetLastError());
-  ctx->nnz = nnz;
-
-  // impact contributions grouped by slot
-  ctx->n_crs = 0;
-  ctx->n_crs_off = 0;
-  if (ctx->n_imp > 0) {
-    const int n = 16 * ctx->n_imp;
-    int *sl0, *sl1, *d_nr, *cnt;
-    uint32_t *cd0;
-    ICF_CUDA(ctx, cudaMallocAsync(&sl0, sizeof(int) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&sl1, sizeof(int) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&cd0, sizeof(uint32_t) * n, s));
-    ICF_CUDA(ctx, cudaMallocAsync(&cnt, sizeof(int) * (n + 1), s));
-    ICF_CUDA(ctx, cudaMallocAsync(&d_nr, sizeof(int), s));
-    if (n + 2 > ctx->cr_cap || !ctx->d_cr) {
-      cudaFree(ctx->d_cr);
-      cudaFree(ctx->d_cr_slot);
-      cudaFree(ctx->d_cr_off);
-      cudaFree(ctx->d_cr_range);
-      cudaFree(ctx->d_cr_pslot);
-      cudaFree(ctx->d_cr_row);
-      ctx->d_cr = nullptr;
-      ctx->d_cr_slot = ctx->d_cr_off = nullptr;
-      ctx->d_cr_range = nullptr;
-      ctx->d_cr_pslot = ctx->d_cr_row = nullptr;
-      const long long cap = 2LL * n + 2;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr, sizeof(uint32_t) * (size_t)cap));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr_slot, sizeof(int) * (size_t)cap));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr_off, sizeof(int) * (size_t)cap));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr_range, sizeof(int2) * (size_t)cap));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr_pslot, sizeof(int) * (size_t)cap));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_cr_row, sizeof(int) * (size_t)cap));
-      ctx->cr_cap = (int)cap;
-    }
-    k_cand_imp_rc<<<icf_blocks(ctx->n_imp, 128), 128, 0, s>>>(ctx->n_imp, ctx->d_imp, ctx->d_alt,
-                                                             ctx->d_mkeys, nnz, sl0, cd0);
-    size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, sl0, sl1, cd0, ctx->d_cr, n, 0, 32, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(ctx->d_tmp, tb, sl0, sl1, cd0, ctx->d_cr, n, 0, 32, s));
-    tb = 0;
-    cub::DeviceRunLengthEncode::Encode(nullptr, tb, sl1, ctx->d_cr_slot, cnt, d_nr, n, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceRunLengthEncode::Encode(ctx->d_tmp, tb, sl1, ctx->d_cr_slot, cnt, d_nr, n, s));
-    int nr = 0;
-    ICF_CUDA(ctx, cudaMemcpyAsync(&nr, d_nr, sizeof(int), cudaMemcpyDeviceToHost, s));
-    ICF_CUDA(ctx, cudaStreamSynchronize(s));
-    // the last run is the invalid slot marker when any candidate was skipped
-    int last = 0;
-    if (nr > 0) {
-      ICF_CUDA(ctx, cudaMemcpyAsync(&last, ctx->d_cr_slot + nr - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-      ICF_CUDA(ctx, cudaStreamSynchronize(s));
-    }
-    const int nvalid = (nr > 0 && last == 0x7fffffff) ? nr - 1 : nr;
-    ICF_CUDA(ctx, cudaMemsetAsync(cnt + nr, 0, sizeof(int), s));
-    tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, ctx->d_cr_off, nr + 1, s);
-    if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-    ICF_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->d_tmp, tb, cnt, ctx->d_cr_off, nr + 1, s));
-    ICF_CUDA(ctx, cudaFreeAsync(sl0, s));
-    ICF_CUDA(ctx, cudaFreeAsync(sl1, s));
-    ICF_CUDA(ctx, cudaFreeAsync(cd0, s));
-    ICF_CUDA(ctx, cudaFreeAsync(cnt, s));
-    ICF_CUDA(ctx, cudaFreeAsync(d_nr, s));
-    ctx->n_crs = nvalid;
-    // where each code's record goes (k_imp_deriv writes, k_imp_add reads)
-    if (n > ctx->imp_pos_cap || !ctx->d_imp_pos) {
-      cudaFree(ctx->d_imp_pos);
-      ctx->d_imp_pos = nullptr;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_imp_pos, sizeof(int) * 2 * (size_t)n));
-      ctx->imp_pos_cap = 2LL * n;
-    }
-    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_imp_pos, 0xFF, sizeof(int) * (size_t)n, s));
-    k_imp_pos<<<icf_blocks(n, 256), 256, 0, s>>>(n, ctx->d_cr_off + nvalid, ctx->d_cr, ctx->d_imp_pos);
-    ICF_CUDA(ctx, cudaGetLastError());
-    // how many of them the off-diagonal gather writes, and the launch order
-    ctx->n_crs_off = 0;
-    if (nvalid > 0) {
-      int *d_flag, *d_pref;
-      ICF_CUDA(ctx, cudaMallocAsync(&d_flag, sizeof(int) * (nvalid + 1LL), s));
-      ICF_CUDA(ctx, cudaMallocAsync(&d_pref, sizeof(int) * (nvalid + 1LL), s));
-      k_flag_off<<<icf_blocks(nvalid + 1LL, 256), 256, 0, s>>>(nvalid, ctx->d_cr_slot, ctx->d_mkeys, ctx->d_src,
-                                                              ctx->src_identity ? 1 : 0, d_flag);
-      tb = 0;
-      cub::DeviceScan::ExclusiveSum(nullptr, tb, d_flag, d_pref, nvalid + 1, s);
-      if (icf_scratch(ctx, tb)) return ICF_ERR_CUDA;
-      ICF_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->d_tmp, tb, d_flag, d_pref, nvalid + 1, s));
-      ICF_CUDA(ctx, cudaMemcpyAsync(&ctx->n_crs_off, d_pref + nvalid, sizeof(int), cudaMemcpyDeviceToHost, s));
-      ICF_CUDA(ctx, cudaStreamSynchronize(s));
-      k_split_off<<<icf_blocks(nvalid, 256), 256, 0, s>>>(nvalid, nvalid - ctx->n_crs_off, ctx->d_cr_slot,
-                                                           ctx->d_cr_off, ctx->d_mkeys, d_pref, ctx->d_cr_range,
-                                                           ctx->d_cr_pslot, ctx->d_cr_row);
-      ICF_CUDA(ctx, cudaGetLastError());
-      ICF_CUDA(ctx, cudaFreeAsync(d_flag, s));
-      ICF_CUDA(ctx, cudaFreeAsync(d_pref, s));
-    }
-    // impact staging
-    if (ctx->n_imp > ctx->ks_cap) {
-      cudaFree(ctx->d_ks);
-      ctx->d_ks = nullptr;
-      const size_t cap = 2 * (size_t)ctx->n_imp;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_ks, sizeof(double) * ICF_IMP_STAGE * cap));
-      ctx->ks_cap = (int)cap;
-    }
-  }
   // outputs
   if ((long long)nnz * 9 > ctx->vals_cap || !ctx->d_vals) {
     cudaFree(ctx->d_vals);
@@ -973,9 +1028,10 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_vals, sizeof(double) * (size_t)c));
     ctx->vals_cap = (int)(c > 0x7fffffff ? 0x7fffffff : c);
   }
-  cudaFree(ctx->d_rhs);
-  ctx->d_rhs = nullptr;
-  ICF_CUDA(ctx, cudaMalloc(&ctx->d_rhs, sizeof(double) * (size_t)(3LL * N + 3)));
+  if (N + 1 > ctx->rhs_rows || !ctx->d_rhs) {
+    ICF_TRY_RC(grow(ctx, &ctx->d_rhs, 3LL * N + 3));
+    ctx->rhs_rows = N + 1;
+  }
   ICF_CUDA(ctx, cudaStreamSynchronize(s));
   return ICF_OK;
 }
