@@ -389,6 +389,7 @@ struct icf_ctx {
   // [5] undecided CZ law comparisons
   int *d_counts = nullptr;
   int *h_counts = nullptr; // pinned
+  bool counts_clean = false;  // d_counts holds zeros once the stream is done
   double *d_norm = nullptr;
   double *h_norm = nullptr; // pinned
 
