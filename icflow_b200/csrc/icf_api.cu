@@ -308,7 +308,7 @@ int icf_set_cz_strength(icf_ctx *ctx, int n_czs, const double *sigma_max, const 
     h[c] = make_double4(sigma_max[c], tau_max[c], dn, dt);
   }
   ICF_TRY(dalloc(ctx, &ctx->d_czprm, (size_t)n_czs));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_czprm, h.data(), sizeof(double4) * (size_t)n_czs, cudaMemcpyHostToDevice));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_czprm, h.data(), sizeof(double4) * (size_t)n_czs));
   ctx->per_cz_prm = true;
   return ICF_OK;
 }
@@ -347,9 +347,9 @@ int icf_cz_law_eval(icf_ctx *ctx, int n, const double *pmax, const double *tmax,
   if (e == cudaSuccess) e = cudaMalloc(&d_out, sizeof(double) * 7 * (size_t)n);
   if (e == cudaSuccess) e = cudaMalloc(&d_fl, sizeof(int) * 3 * (size_t)n);
   if (e == cudaSuccess && strength) e = cudaMalloc(&d_prm, sizeof(double4) * (size_t)n);
-  if (e == cudaSuccess) e = cudaMemcpy(d_in, in.data(), sizeof(double) * in.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = icf_h2d(ctx->stream, d_in, in.data(), sizeof(double) * in.size());
   if (e == cudaSuccess && strength)
-    e = cudaMemcpy(d_prm, prm.data(), sizeof(double4) * prm.size(), cudaMemcpyHostToDevice);
+    e = icf_h2d(ctx->stream, d_prm, prm.data(), sizeof(double4) * prm.size());
   if (e == cudaSuccess) rc = icf_launch_law_eval(ctx, n, d_in, d_prm, d_out, d_fl);
   std::vector<double> out;
   std::vector<int> fl;
@@ -490,9 +490,9 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
 
   std::vector<double4> hx(n);
   for (size_t i = 0; i < n; i++) hx[i] = make_double4(x0[3 * i], x0[3 * i + 1], x0[3 * i + 2], 0.0);
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_alt, alt_id, sizeof(int) * n, cudaMemcpyHostToDevice));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_x0, hx.data(), sizeof(double4) * n, cudaMemcpyHostToDevice));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_xc, hx.data(), sizeof(double4) * n, cudaMemcpyHostToDevice));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_alt, alt_id, sizeof(int) * n));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_x0, hx.data(), sizeof(double4) * n));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_xc, hx.data(), sizeof(double4) * n));
   ICF_CUDA(ctx, cudaMemset(ctx->d_va, 0, sizeof(double2) * 3 * n));
   ICF_CUDA(ctx, cudaMemset(ctx->d_u, 0, sizeof(double) * 3 * n));
   ICF_CUDA(ctx, cudaMemset(ctx->d_v, 0, sizeof(double) * 3 * n));
@@ -501,12 +501,12 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
   ICF_CUDA(ctx, cudaMemset(ctx->d_un, 0, sizeof(double) * 3 * n));
   ICF_CUDA(ctx, cudaMemset(ctx->d_nodeF, 0, sizeof(double) * 3 * n));
   if (n_elems)
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_elem, elems, sizeof(int4) * (size_t)n_elems, cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_elem, elems, sizeof(int4) * (size_t)n_elems));
   if (n_czs) {
     std::vector<int> hc(8 * (size_t)n_czs, 0);
     for (int c = 0; c < n_czs; c++)
       for (int i = 0; i < 6; i++) hc[8 * (size_t)c + i] = czs[6 * (size_t)c + i];
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_cz, hc.data(), sizeof(int) * hc.size(), cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_cz, hc.data(), sizeof(int) * hc.size()));
     ICF_CUDA(ctx, cudaMemset(ctx->d_czs, 0, sizeof(double) * 8 * (size_t)n_czs));
     ICF_CUDA(ctx, cudaMemset(ctx->d_czfail, 0, sizeof(int) * (size_t)n_czs));
     ICF_CUDA(ctx, cudaMemset(ctx->d_cztent, 0, sizeof(double) * 2 * (size_t)n_czs));
@@ -518,11 +518,11 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
     ICF_TRY(dalloc(ctx, &ctx->d_adj_off, (size_t)n_surface + 1));
     ICF_TRY(dalloc(ctx, &ctx->d_adj, (size_t)adj_offsets[n_surface]));
     ICF_TRY(dalloc(ctx, &ctx->d_faces, 3 * (size_t)n_faces));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_selem, surface_elems, sizeof(int4) * (size_t)n_surface, cudaMemcpyHostToDevice));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_adj_off, adj_offsets, sizeof(int) * ((size_t)n_surface + 1), cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_selem, surface_elems, sizeof(int4) * (size_t)n_surface));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_adj_off, adj_offsets, sizeof(int) * ((size_t)n_surface + 1)));
     if (adj_offsets[n_surface] > 0)
-      ICF_CUDA(ctx, cudaMemcpy(ctx->d_adj, adj_faces, sizeof(int) * (size_t)adj_offsets[n_surface], cudaMemcpyHostToDevice));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_faces, faces, sizeof(int) * 3 * (size_t)n_faces, cudaMemcpyHostToDevice));
+      ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_adj, adj_faces, sizeof(int) * (size_t)adj_offsets[n_surface]));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_faces, faces, sizeof(int) * 3 * (size_t)n_faces));
     // surface nodes and the surface elements holding each (counting sort by
     // node: ascending nodes, ascending elements per node)
     std::vector<int> cnt(n + 1, 0);
@@ -553,9 +553,9 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
     ICF_TRY(dalloc(ctx, &ctx->d_snode, snode.size()));
     ICF_TRY(dalloc(ctx, &ctx->d_sinc_off, off2.size()));
     ICF_TRY(dalloc(ctx, &ctx->d_sinc, inc2.size()));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_snode, snode.data(), sizeof(int) * snode.size(), cudaMemcpyHostToDevice));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_sinc_off, off2.data(), sizeof(int) * off2.size(), cudaMemcpyHostToDevice));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_sinc, inc2.data(), sizeof(int) * inc2.size(), cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_snode, snode.data(), sizeof(int) * snode.size()));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_sinc_off, off2.data(), sizeof(int) * off2.size()));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_sinc, inc2.data(), sizeof(int) * inc2.size()));
   }
   ctx->have_static = true;
   ctx->version++;
@@ -593,8 +593,8 @@ int icf_transfer_cz_state(icf_ctx *ctx, int n_czs, const double *pmax, const dou
       h[8 * (size_t)c + 3 + i] = tmax[3 * (size_t)c + i];
     }
   if (n_czs) {
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_czs, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_czfail, failed, sizeof(int) * (size_t)n_czs, cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_czs, h.data(), sizeof(double) * h.size()));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_czfail, failed, sizeof(int) * (size_t)n_czs));
   }
   return ICF_OK;
 }
@@ -608,7 +608,7 @@ int icf_set_surface_groups(icf_ctx *ctx, int n_surface, const int *group) {
   if (!group) return ICF_OK;
   if (n_surface != ctx->n_surf) return icf_fail(ctx, ICF_ERR_ARG, "n_surface does not match the static data");
   ICF_TRY(dalloc(ctx, &ctx->d_sgroup, (size_t)n_surface));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_sgroup, group, sizeof(int) * (size_t)n_surface, cudaMemcpyHostToDevice));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_sgroup, group, sizeof(int) * (size_t)n_surface));
   // bits of the largest group id (for the broad phase's (cell, group) keys);
   // -1 when some id is negative
   int gmax = 0;
@@ -743,7 +743,7 @@ int icf_set_impacts(icf_ctx *ctx, int n_impacts, const int *impacts) {
     ctx->imp_gen++;
   }
   if (n_impacts)
-    ICF_CUDA(ctx, cudaMemcpy(ctx->d_imp, impacts, sizeof(int4) * (size_t)n_impacts, cudaMemcpyHostToDevice));
+    ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_imp, impacts, sizeof(int4) * (size_t)n_impacts));
   ctx->n_imp = n_impacts;
   ctx->imp_cmp_valid = false;
   ctx->have_structure = false;
@@ -1027,9 +1027,9 @@ int icf_set_node_state(icf_ctx *ctx, int n_nodes, const double *u, const double 
   if (!ctx->have_static) return icf_fail(ctx, ICF_ERR_STATE, "icf_transfer_static first");
   if (n_nodes != ctx->n_nodes || !u || !v || !a) return icf_fail(ctx, ICF_ERR_ARG, "bad node arrays");
   const size_t b = sizeof(double) * 3 * (size_t)n_nodes;
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_u, u, b, cudaMemcpyHostToDevice));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_v, v, b, cudaMemcpyHostToDevice));
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_a, a, b, cudaMemcpyHostToDevice));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_u, u, b));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_v, v, b));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_a, a, b));
   return ICF_OK;
 }
 
@@ -1047,7 +1047,7 @@ int icf_get_node_state(icf_ctx *ctx, double *u, double *v, double *a, double *du
 int icf_set_du(icf_ctx *ctx, int n_nodes, const double *du) {
   ICF_CHECK_CTX(ctx);
   if (n_nodes != ctx->n_nodes || !du) return icf_fail(ctx, ICF_ERR_ARG, "bad du array");
-  ICF_CUDA(ctx, cudaMemcpy(ctx->d_du, du, sizeof(double) * 3 * (size_t)n_nodes, cudaMemcpyHostToDevice));
+  ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_du, du, sizeof(double) * 3 * (size_t)n_nodes));
   return ICF_OK;
 }
 

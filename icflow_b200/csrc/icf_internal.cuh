@@ -494,6 +494,14 @@ int icf_fail(icf_ctx *ctx, int code, const std::string &msg);
                       std::string(#call) + ": " + cudaGetErrorString(e_));     \
   } while (0)
 
+// A host-to-device copy that the work enqueued on s afterwards sees whole.  The
+// plain copy may return while the last of a pageable buffer is still on its way,
+// and a non-blocking stream does not wait for it.
+inline cudaError_t icf_h2d(cudaStream_t s, void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 int icf_scratch(icf_ctx *ctx, size_t bytes);
 #define ICF_TRY_RC(call)        \
   do {                          \

@@ -232,7 +232,7 @@ int icf_build_tiles(icf_ctx *ctx) {
   auto up = [&](auto **d, const auto &h) -> int {
     typedef typename std::decay<decltype(h[0])>::type E;
     ICF_CUDA(ctx, cudaMalloc(d, sizeof(E) * std::max<size_t>(h.size(), 1)));
-    if (!h.empty()) ICF_CUDA(ctx, cudaMemcpy(*d, h.data(), sizeof(E) * h.size(), cudaMemcpyHostToDevice));
+    if (!h.empty()) ICF_CUDA(ctx, icf_h2d(ctx->stream, *d, h.data(), sizeof(E) * h.size()));
     return ICF_OK;
   };
   ICF_TRY_RC(up(&T.tiles, h_tiles));
