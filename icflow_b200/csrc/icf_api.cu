@@ -493,13 +493,15 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
   ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_alt, alt_id, sizeof(int) * n));
   ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_x0, hx.data(), sizeof(double4) * n));
   ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_xc, hx.data(), sizeof(double4) * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_va, 0, sizeof(double2) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_u, 0, sizeof(double) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_v, 0, sizeof(double) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_a, 0, sizeof(double) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_du, 0, sizeof(double) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_un, 0, sizeof(double) * 3 * n));
-  ICF_CUDA(ctx, cudaMemset(ctx->d_nodeF, 0, sizeof(double) * 3 * n));
+  // on the stream of the copies that later calls make into these arrays: a fill
+  // on the null stream could still run after them
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_va, 0, sizeof(double2) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_u, 0, sizeof(double) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_v, 0, sizeof(double) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_a, 0, sizeof(double) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_du, 0, sizeof(double) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_un, 0, sizeof(double) * 3 * n, ctx->stream));
+  ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_nodeF, 0, sizeof(double) * 3 * n, ctx->stream));
   if (n_elems)
     ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_elem, elems, sizeof(int4) * (size_t)n_elems));
   if (n_czs) {
@@ -507,11 +509,11 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
     for (int c = 0; c < n_czs; c++)
       for (int i = 0; i < 6; i++) hc[8 * (size_t)c + i] = czs[6 * (size_t)c + i];
     ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_cz, hc.data(), sizeof(int) * hc.size()));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_czs, 0, sizeof(double) * 8 * (size_t)n_czs));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_czfail, 0, sizeof(int) * (size_t)n_czs));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_cztent, 0, sizeof(double) * 2 * (size_t)n_czs));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_czflags, 0, sizeof(int) * (size_t)n_czs));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_czavg, 0, sizeof(double) * 4 * (size_t)n_czs));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_czs, 0, sizeof(double) * 8 * (size_t)n_czs, ctx->stream));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_czfail, 0, sizeof(int) * (size_t)n_czs, ctx->stream));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_cztent, 0, sizeof(double) * 2 * (size_t)n_czs, ctx->stream));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_czflags, 0, sizeof(int) * (size_t)n_czs, ctx->stream));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_czavg, 0, sizeof(double) * 4 * (size_t)n_czs, ctx->stream));
   }
   if (n_surface) {
     ICF_TRY(dalloc(ctx, &ctx->d_selem, (size_t)n_surface));

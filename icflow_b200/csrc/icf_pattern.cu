@@ -615,9 +615,9 @@ int icf_build_static_pattern(icf_ctx *ctx) {
     ctx->N = 0;
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_skeys, sizeof(unsigned long long)));
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_rc_off, sizeof(int)));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_rc_off, 0, sizeof(int)));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_rc_off, 0, sizeof(int), s));
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_srow, sizeof(int)));
-    ICF_CUDA(ctx, cudaMemset(ctx->d_srow, 0, sizeof(int)));
+    ICF_CUDA(ctx, cudaMemsetAsync(ctx->d_srow, 0, sizeof(int), s));
     return ICF_OK;
   }
   unsigned long long *k0, *k1;
