@@ -592,12 +592,15 @@ int icf_mlp_create(int device, icf_mlp **out) {
   std::vector<float> norm(2 * NI + NO, 0.f);
   for (int i = 0; i < NI; i++) norm[NI + i] = 1.f;
   for (int i = 0; i < NO; i++) norm[2 * NI + i] = 1.f;
-  cudaMemcpy(m->d_norm, norm.data(), sizeof(float) * norm.size(), cudaMemcpyHostToDevice);
-  cudaMemset(m->d_master, 0, sizeof(float) * NPAR);
-  cudaMemset(m->d_m, 0, sizeof(float) * NPAR);
-  cudaMemset(m->d_v, 0, sizeof(float) * NPAR);
-  k_mlp_pack<<<icf_blocks(WB_N, 256), 256, 0, m->stream>>>(m->d_master, m->d_wb);
-  if (cudaStreamSynchronize(m->stream) != cudaSuccess) {
+  // (copies and fills on the network's stream, here and below: the null stream
+  // is not ordered with it)
+  cudaStream_t s = m->stream;
+  icf_h2d(s, m->d_norm, norm.data(), sizeof(float) * norm.size());
+  cudaMemsetAsync(m->d_master, 0, sizeof(float) * NPAR, s);
+  cudaMemsetAsync(m->d_m, 0, sizeof(float) * NPAR, s);
+  cudaMemsetAsync(m->d_v, 0, sizeof(float) * NPAR, s);
+  k_mlp_pack<<<icf_blocks(WB_N, 256), 256, 0, s>>>(m->d_master, m->d_wb);
+  if (cudaStreamSynchronize(s) != cudaSuccess) {
     delete m;
     return ICF_ERR_CUDA;
   }
@@ -622,13 +625,14 @@ int icf_mlp_param_count(void) { return NPAR; }
 int icf_mlp_set_params(icf_mlp *m, const float *params, const float *norm) {
   if (!m || !params) return ICF_ERR_ARG;
   MLP_CUDA(m, cudaSetDevice(m->device));
-  MLP_CUDA(m, cudaMemcpy(m->d_master, params, sizeof(float) * NPAR, cudaMemcpyHostToDevice));
-  if (norm) MLP_CUDA(m, cudaMemcpy(m->d_norm, norm, sizeof(float) * (2 * NI + NO), cudaMemcpyHostToDevice));
-  MLP_CUDA(m, cudaMemset(m->d_m, 0, sizeof(float) * NPAR));
-  MLP_CUDA(m, cudaMemset(m->d_v, 0, sizeof(float) * NPAR));
+  cudaStream_t s = m->stream;
+  MLP_CUDA(m, icf_h2d(s, m->d_master, params, sizeof(float) * NPAR));
+  if (norm) MLP_CUDA(m, icf_h2d(s, m->d_norm, norm, sizeof(float) * (2 * NI + NO)));
+  MLP_CUDA(m, cudaMemsetAsync(m->d_m, 0, sizeof(float) * NPAR, s));
+  MLP_CUDA(m, cudaMemsetAsync(m->d_v, 0, sizeof(float) * NPAR, s));
   m->adam_t = 0;
-  k_mlp_pack<<<icf_blocks(WB_N, 256), 256, 0, m->stream>>>(m->d_master, m->d_wb);
-  MLP_CUDA(m, cudaStreamSynchronize(m->stream));
+  k_mlp_pack<<<icf_blocks(WB_N, 256), 256, 0, s>>>(m->d_master, m->d_wb);
+  MLP_CUDA(m, cudaStreamSynchronize(s));
   return ICF_OK;
 }
 
@@ -738,8 +742,8 @@ int icf_mlp_train(icf_mlp *m, int n, const float *x, const float *y, int epochs,
   MLP_CUDA(m, cudaMalloc(&dx_all, sizeof(float) * NI * (size_t)n));
   MLP_CUDA(m, cudaMalloc(&dy_all, sizeof(float) * NO * (size_t)n));
   MLP_CUDA(m, cudaMalloc(&d_order, sizeof(int) * (size_t)n));
-  MLP_CUDA(m, cudaMemcpy(dx_all, x, sizeof(float) * NI * (size_t)n, cudaMemcpyHostToDevice));
-  MLP_CUDA(m, cudaMemcpy(dy_all, y, sizeof(float) * NO * (size_t)n, cudaMemcpyHostToDevice));
+  MLP_CUDA(m, icf_h2d(s, dx_all, x, sizeof(float) * NI * (size_t)n));
+  MLP_CUDA(m, icf_h2d(s, dy_all, y, sizeof(float) * NO * (size_t)n));
   std::vector<int> order(n);
   for (int i = 0; i < n; i++) order[i] = i;
   unsigned long long st = seed * 6364136223846793005ull + 1442695040888963407ull;

@@ -2,7 +2,7 @@
 runs on a stream of its own that does not wait for the null stream, and a copy
 from pageable memory or a fill on the null stream may return before it has run:
 neither may be used in the library, and work pending on the default stream of
-the host program changes no result."""
+the host program changes no result.  A network's stream is of the same kind."""
 import re
 from pathlib import Path
 
@@ -14,7 +14,7 @@ from icflow_b200.model_prms import config_prms
 from tests.harness import random_state
 
 CSRC = Path(__file__).resolve().parents[1] / "icflow_b200" / "csrc"
-SOURCES = sorted(p.name for p in [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")] if p.name != "icf_mlp.cu")
+SOURCES = sorted(p.name for p in [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")])
 
 
 @pytest.mark.parametrize("name", SOURCES)
@@ -79,3 +79,30 @@ def test_static_data_under_pending_work():
     a, b = _values(coll, False), _values(coll, True)
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+def _network(busy):
+    from icflow_b200.warm_start import MLP, NI, NO, init_params
+
+    rng = np.random.default_rng(4)
+    p, norm = init_params(1), np.concatenate([rng.normal(size=NI), rng.uniform(0.5, 2, NI), np.ones(NO)])
+    x = rng.normal(size=(5000, NI)).astype(np.float32)
+    t = rng.normal(size=(5000, NO)).astype(np.float32)
+    keep = pending_work() if busy else None
+    net = MLP()
+    net.set_params(p, norm.astype(np.float32))
+    g0, l0 = net.grad(x, t)
+    loss = net.train(x, t, epochs=2, batch=512, lr=1e-3, seed=3)
+    q = net.get_params()[0]
+    net.set_params(p, norm.astype(np.float32))  # and the moments start from zero again
+    again = net.train(x, t, epochs=2, batch=512, lr=1e-3, seed=3)
+    net.close()
+    del keep
+    assert loss == again
+    return g0, l0, loss, q
+
+
+@pytest.mark.gpu
+def test_network_under_pending_work():
+    for a, b in zip(_network(False), _network(True)):
+        assert np.array_equal(a, b)
