@@ -430,7 +430,8 @@ int icf_transfer_static(icf_ctx *ctx, int n_nodes, const double *x0, const int *
   ctx->d_imp = nullptr; ctx->imp_cap = 0; ctx->n_imp = 0;
   ctx->d_cr_range = nullptr; ctx->d_cr_pslot = ctx->d_cr_row = nullptr;
   ctx->cr_cap = 0; ctx->n_crs = 0; ctx->d_pairs = ctx->d_masks = nullptr;
-  ctx->pairs_cap = 0; ctx->n_pairs = 0; ctx->d_vals = ctx->d_rhs = ctx->d_nodeF = nullptr; ctx->vals_cap = ctx->rhs_rows = 0;
+  ctx->pairs_cap = 0; ctx->n_pairs = 0; ctx->d_vals = ctx->d_rhs = ctx->d_nodeF = nullptr; ctx->vals_cap = 0;
+  ctx->rhs_cap = 0;
   ctx->tet_inc = icf_node_inc(); ctx->imp_inc = icf_node_inc(); ctx->d_tmp = nullptr; ctx->tmp_bytes = 0;
   ctx->sell_off = icf_sell();
   ctx->sell_diag = icf_sell();

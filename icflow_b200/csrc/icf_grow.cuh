@@ -1,0 +1,19 @@
+// icf_grow.cuh -- device arrays that share one capacity.  Over an allocator `Mem`
+// with alloc(void **, bytes) -> success and free(void *), so that it compiles
+// without CUDA as well.
+#pragma once
+#include <cstddef>
+
+// Arrays of n elements each in place of the ones at *p, whose contents are not
+// kept.  The capacity holds for all of them: it is zero from the first release
+// until the last allocation has succeeded, so that after a failure the next call
+// allocates all of them again, however few elements it needs.
+template <class Mem, class Cap, class... T>
+bool icf_grow_all(Mem &mem, Cap *cap, long long n, T **...p) {
+  *cap = 0;
+  ((mem.free(*p), *p = nullptr), ...);
+  bool ok = true;
+  ((ok = ok && mem.alloc(reinterpret_cast<void **>(p), sizeof(T) * (size_t)n)), ...);
+  if (ok) *cap = (Cap)n;
+  return ok;
+}

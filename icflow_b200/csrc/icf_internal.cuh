@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/icflow_b200.h"
+#include "icf_grow.cuh"
 
 #define ICF_KIND_TET 0u
 #define ICF_KIND_CZ 1u
@@ -288,7 +289,7 @@ struct icf_ctx {
   double4 *d_es = nullptr;
   double *d_cs = nullptr;
   double *d_ks = nullptr;
-  int ks_cap = 0;
+  long long ks_cap = 0;  // doubles of d_ks
 
   // static pattern
   unsigned long long *d_skeys = nullptr;
@@ -350,7 +351,7 @@ struct icf_ctx {
   int imp_differ = 1;
   icf_contact_ws cws;
   // per-impact classification {kind, ia, ib, 0} and {s, t, dsq, 0}; same
-  // capacity as the impact staging d_ks (ks_cap)
+  // capacity as the impact staging d_ks
   int n_crs = 0;                  // slots touched by impacts
   int cr_cap = 0;
   // the touched slots in k_imp_add's order: those the off-diagonal gather
@@ -383,7 +384,8 @@ struct icf_ctx {
 
   // outputs
   double *d_vals = nullptr, *d_rhs = nullptr, *d_nodeF = nullptr;
-  int vals_cap = 0, rhs_rows = 0;
+  int vals_cap = 0;
+  long long rhs_cap = 0;
 
   // counters: [0] damaged [1] failed [2] contact [3] active impacts [4] nonfinite
   // [5] undecided CZ law comparisons
@@ -503,6 +505,25 @@ inline cudaError_t icf_h2d(cudaStream_t s, void *dst, const void *src, size_t by
 }
 
 int icf_scratch(icf_ctx *ctx, size_t bytes);
+
+// Device memory as icf_grow_all takes it.  A failure leaves no error behind for
+// the check of a later launch to find.
+struct icf_device_mem {
+  cudaError_t err = cudaSuccess;
+  bool alloc(void **p, size_t bytes) {
+    err = cudaMalloc(p, bytes);
+    if (err != cudaSuccess) cudaGetLastError();
+    return err == cudaSuccess;
+  }
+  void free(void *p) { cudaFree(p); }
+};
+// n elements for each of the arrays that share the capacity *cap
+template <class Cap, class... T>
+int icf_grow(icf_ctx *ctx, Cap *cap, long long n, T **...p) {
+  icf_device_mem mem;
+  if (icf_grow_all(mem, cap, n, p...)) return ICF_OK;
+  return icf_fail(ctx, ICF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(mem.err));
+}
 #define ICF_TRY_RC(call)        \
   do {                          \
     const int rc_ = (call);     \

@@ -883,14 +883,6 @@ static int build_lists(icf_ctx *ctx, bool off, bool diag) {
   return ICF_OK;
 }
 
-template <typename T>
-static int grow(icf_ctx *ctx, T **p, long long n) {
-  cudaFree(*p);
-  *p = nullptr;
-  ICF_CUDA(ctx, cudaMalloc(p, sizeof(T) * (size_t)n));
-  return ICF_OK;
-}
-
 void icf_free_dyn_ws(icf_ctx *ctx) {
   icf_dyn_ws &D = ctx->dyn;
   void *ptrs[] = {D.cnt, D.off, D.stat, D.pre, D.items, D.newcol, D.small};
@@ -907,26 +899,13 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
   if (ni > 0) {
     // per-row work arrays (cnt stays zero between builds) and the items
     if (N + 1 > D.rows_cap) {
-      const long long c = N + 1LL;
-      ICF_TRY_RC(grow(ctx, &D.cnt, c));
-      ICF_TRY_RC(grow(ctx, &D.off, c));
-      ICF_TRY_RC(grow(ctx, &D.stat, c));
-      ICF_TRY_RC(grow(ctx, &D.pre, c));
-      ICF_CUDA(ctx, cudaMemsetAsync(D.cnt, 0, sizeof(int) * (size_t)c, s));
       if (!D.small) ICF_CUDA(ctx, cudaMalloc(&D.small, sizeof(int)));
       if (!D.h_small) ICF_CUDA(ctx, cudaMallocHost(&D.h_small, 8 * sizeof(int)));
-      D.rows_cap = N + 1;
+      ICF_TRY_RC(icf_grow(ctx, &D.rows_cap, N + 1LL, &D.cnt, &D.off, &D.stat, &D.pre));
+      ICF_CUDA(ctx, cudaMemsetAsync(D.cnt, 0, sizeof(int) * (N + 1LL), s));
     }
-    if (16LL * ni > D.items_cap) {
-      const long long c = 16LL * ni + 4LL * ni;
-      ICF_TRY_RC(grow(ctx, &D.items, c));
-      ICF_TRY_RC(grow(ctx, &D.newcol, c));
-      D.items_cap = c;
-    }
-    if (16LL * ni > ctx->imp_pos_cap || !ctx->d_imp_pos) {
-      ICF_TRY_RC(grow(ctx, &ctx->d_imp_pos, 32LL * ni));
-      ctx->imp_pos_cap = 32LL * ni;
-    }
+    if (16LL * ni > D.items_cap) ICF_TRY_RC(icf_grow(ctx, &D.items_cap, 20LL * ni, &D.items, &D.newcol));
+    if (16LL * ni > ctx->imp_pos_cap) ICF_TRY_RC(icf_grow(ctx, &ctx->imp_pos_cap, 32LL * ni, &ctx->d_imp_pos));
     size_t tb = 0, tb2 = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, D.cnt, D.off, N + 1, s);
     cub::DeviceScan::ExclusiveScan(nullptr, tb2, D.stat, D.pre, int4_sum(), make_int4(0, 0, 0, 0), N + 1, s);
@@ -948,34 +927,20 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
     tot = make_int4(D.h_small[0], D.h_small[1], D.h_small[2], 0);
   }
   const int nd = tot.x, nnz = nnz_s + nd;
-  if (nnz + 1 > ctx->cols_cap || !ctx->d_cols) {
-    const long long cap = nnz + 1 + nnz / 8 + 64;
-    ICF_TRY_RC(grow(ctx, &ctx->d_cols, cap));
-    ICF_TRY_RC(grow(ctx, &ctx->d_mkeys, cap));
-    ctx->cols_cap = (int)cap;
-  }
-  if (N + 1 > ctx->rows_cap || !ctx->d_rows) {
-    ICF_TRY_RC(grow(ctx, &ctx->d_rows, N + 1LL));
-    ctx->rows_cap = N + 1;
-  }
+  if (nnz + 1 > ctx->cols_cap)
+    ICF_TRY_RC(icf_grow(ctx, &ctx->cols_cap, nnz + 1LL + nnz / 8 + 64, &ctx->d_cols, &ctx->d_mkeys));
+  if (N + 1 > ctx->rows_cap) ICF_TRY_RC(icf_grow(ctx, &ctx->rows_cap, N + 1LL, &ctx->d_rows));
   if (ni == 0) {
     ICF_CUDA(ctx, cudaMemcpyAsync(ctx->d_mkeys, ctx->d_skeys, sizeof(unsigned long long) * (size_t)nnz_s,
                                   cudaMemcpyDeviceToDevice, s));
     if (nnz > 0) k_cols<<<icf_blocks(nnz, 256), 256, 0, s>>>(nnz, ctx->d_mkeys, ctx->d_cols);
     k_rows<<<icf_blocks((long long)N + 1, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, ctx->d_rows);
   } else {
-    if (!ctx->d_s2m || ctx->s2m_cap < nnz_s + 1) {
-      ICF_TRY_RC(grow(ctx, &ctx->d_s2m, nnz_s + 1LL));
-      ctx->s2m_cap = nnz_s + 1;
-    }
+    if (nnz_s + 1 > ctx->s2m_cap) ICF_TRY_RC(icf_grow(ctx, &ctx->s2m_cap, nnz_s + 1LL, &ctx->d_s2m));
     const int n_crs = tot.y + tot.z;
-    if (n_crs > ctx->cr_cap || !ctx->d_cr_range) {
-      const long long c = n_crs + n_crs / 4 + 16;
-      ICF_TRY_RC(grow(ctx, &ctx->d_cr_range, c));
-      ICF_TRY_RC(grow(ctx, &ctx->d_cr_pslot, c));
-      ICF_TRY_RC(grow(ctx, &ctx->d_cr_row, c));
-      ctx->cr_cap = (int)c;
-    }
+    if (n_crs + 1 > ctx->cr_cap)
+      ICF_TRY_RC(icf_grow(ctx, &ctx->cr_cap, n_crs + n_crs / 4 + 16LL, &ctx->d_cr_range, &ctx->d_cr_pslot,
+                          &ctx->d_cr_row));
     k_imp_write<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, tot.y, D.off, D.items, ctx->d_srow, ctx->d_skeys,
                                                               D.pre, ctx->d_rows, ctx->d_mkeys, ctx->d_cols, D.newcol,
                                                               ctx->d_imp_pos, ctx->d_cr_range, ctx->d_cr_pslot,
@@ -984,10 +949,8 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
       k_merge_static<<<icf_blocks(nnz_s, 256), 256, 0, s>>>(nnz_s, ctx->d_skeys, D.pre, D.newcol, ctx->d_mkeys,
                                                            ctx->d_cols, ctx->d_s2m);
     // impact staging
-    if (ni > ctx->ks_cap) {
-      ICF_TRY_RC(grow(ctx, &ctx->d_ks, (long long)ICF_IMP_STAGE * 2 * ni));
-      ctx->ks_cap = 2 * ni;
-    }
+    if ((long long)ICF_IMP_STAGE * ni > ctx->ks_cap)
+      ICF_TRY_RC(icf_grow(ctx, &ctx->ks_cap, (long long)ICF_IMP_STAGE * 2 * ni, &ctx->d_ks));
   }
   ICF_CUDA(ctx, cudaGetLastError());
   ctx->src_identity = nd == 0;
@@ -1028,10 +991,7 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
     ICF_CUDA(ctx, cudaMalloc(&ctx->d_vals, sizeof(double) * (size_t)c));
     ctx->vals_cap = (int)(c > 0x7fffffff ? 0x7fffffff : c);
   }
-  if (N + 1 > ctx->rhs_rows || !ctx->d_rhs) {
-    ICF_TRY_RC(grow(ctx, &ctx->d_rhs, 3LL * N + 3));
-    ctx->rhs_rows = N + 1;
-  }
+  if (3LL * N + 3 > ctx->rhs_cap) ICF_TRY_RC(icf_grow(ctx, &ctx->rhs_cap, 3LL * N + 3, &ctx->d_rhs));
   ICF_CUDA(ctx, cudaStreamSynchronize(s));
   return ICF_OK;
 }

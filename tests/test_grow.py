@@ -1,0 +1,82 @@
+"""The growth of device arrays when allocations fail, over an allocator that
+fails where it is told to (compiled here with g++; no GPU): whatever fails, no
+capacity claims an array that is not there, and the next call makes up for it."""
+import re
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "icflow_b200" / "csrc"
+
+PROBE = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include "icf_grow.cuh"
+
+struct fake {
+  int fail_at = -1, calls = 0;
+  std::map<void *, size_t> live;
+  bool alloc(void **p, size_t bytes) {
+    if (calls++ == fail_at) return false;
+    *p = std::malloc(bytes);
+    live[*p] = bytes;
+    return true;
+  }
+  void free(void *p) {
+    if (!p) return;
+    if (!live.erase(p)) std::abort();
+    std::free(p);
+  }
+};
+
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } } while (0)
+
+int main() {
+  for (int fail = -1; fail < 3; fail++) {
+    fake m;
+    int *a = nullptr;
+    double *b = nullptr;
+    char *c = nullptr;
+    long long cap = 0;
+    auto have = [&](long long n) {  // what a call that needs n elements finds
+      if (n > cap && !icf_grow_all(m, &cap, n, &a, &b, &c)) return false;
+      CHECK(m.live.count(a) && m.live[a] >= sizeof(int) * n);
+      CHECK(m.live.count(b) && m.live[b] >= sizeof(double) * n);
+      CHECK(m.live.count(c) && m.live[c] >= (size_t)n);
+      return true;
+    };
+    CHECK(have(100) && cap == 100);
+    CHECK(have(40) && cap == 100 && m.calls == 3);
+    m.fail_at = fail < 0 ? -1 : m.calls + fail;
+    CHECK(have(1000) == (fail < 0));
+    if (fail >= 0) CHECK(cap == 0);
+    m.fail_at = -1;
+    CHECK(have(40));  // fewer than before the failure
+    CHECK(have(1000) && cap == 1000);
+    int small_cap = 7;
+    CHECK(icf_grow_all(m, &small_cap, 50, &a) && small_cap == 50);
+  }
+  return 0;
+}
+"""
+
+
+def test_failed_allocations(tmp_path):
+    if not shutil.which("g++"):
+        pytest.skip("g++ not available")
+    (tmp_path / "probe.cpp").write_text(PROBE)
+    exe = tmp_path / "probe"
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-I", str(CSRC), str(tmp_path / "probe.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
+
+
+def test_arrays_of_one_capacity_grow_together():
+    """The capacities of the structure's merge are set by the growth of their
+    arrays, never by hand."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "icf_pattern.cu").read_text())
+    caps = "rows_cap|items_cap|cols_cap|cr_cap|ks_cap|imp_pos_cap|s2m_cap|rhs_cap"
+    assert not re.findall(rf"\b(?:{caps})\s*=[^=]", text)
