@@ -1,6 +1,7 @@
-// icf_grow.cuh -- device arrays that share one capacity.  Over an allocator `Mem`
-// with alloc(void **, bytes) -> success and free(void *), so that it compiles
-// without CUDA as well.
+// icf_grow.cuh -- device arrays that share one capacity, and temporaries that
+// return to their allocator whichever way a function ends.  Over an allocator
+// `Mem` with alloc(void **, bytes) -> success and free(void *), so that it
+// compiles without CUDA as well.
 #pragma once
 #include <cstddef>
 
@@ -17,3 +18,23 @@ bool icf_grow_all(Mem &mem, Cap *cap, long long n, T **...p) {
   if (ok) *cap = (Cap)n;
   return ok;
 }
+
+// Temporaries: alloc() registers what it gave, the destructor frees it.
+template <class Mem, int MAX = 8>
+struct icf_temps {
+  Mem &mem;
+  void *held[MAX] = {};
+  int n = 0;
+  explicit icf_temps(Mem &m) : mem(m) {}
+  icf_temps(const icf_temps &) = delete;
+  ~icf_temps() {
+    while (n > 0) mem.free(held[--n]);
+  }
+  template <class T>
+  bool alloc(T **p, long long count) {
+    *p = nullptr;
+    if (n == MAX || !mem.alloc(reinterpret_cast<void **>(p), sizeof(T) * (size_t)count)) return false;
+    held[n++] = *p;
+    return true;
+  }
+};

@@ -195,7 +195,8 @@ struct icf_solver {
       *hcol = nullptr;
   unsigned short *eidx = nullptr;
   unsigned char *last = nullptr;
-  long long sstep_cap = 0, eslot_cap = 0, ecol_cap = 0, eidx_cap = 0, last_cap = 0, n_steps = 0;
+  long long sstep_cap = 0, eslot_cap = 0, ecol_cap = 0, eidx_cap = 0, last_cap = 0, part_cap = 0, hcol_cap = 0,
+            n_steps = 0;
   int blocks = 0;
   bool halo = false;
   int most[3] = {0, 0, 0};  // rows and halo of the largest thread block, batches of the largest warp
@@ -516,6 +517,16 @@ struct icf_device_mem {
     return err == cudaSuccess;
   }
   void free(void *p) { cudaFree(p); }
+};
+// Temporaries of a stream, from the device's memory pool.
+struct icf_stream_mem {
+  cudaStream_t s;
+  bool alloc(void **p, size_t bytes) {
+    const bool ok = cudaMallocAsync(p, bytes, s) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  }
+  void free(void *p) { cudaFreeAsync(p, s); }
 };
 // n elements for each of the arrays that share the capacity *cap
 template <class Cap, class... T>

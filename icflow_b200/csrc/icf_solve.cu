@@ -888,14 +888,13 @@ __global__ void __launch_bounds__(MR_THREADS, 1) k_minres(const mr_args A) {
 
 template <typename T>
 int grow(icf_ctx *ctx, T **p, long long *cap, long long n) {
-  if (n <= *cap && *p) return ICF_OK;
-  cudaFree(*p);
-  *p = nullptr;
-  const long long c = n + n / 4 + 16;
-  ICF_CUDA(ctx, cudaMalloc(p, sizeof(T) * (size_t)c));
-  *cap = c;
-  return ICF_OK;
+  return n <= *cap ? ICF_OK : icf_grow(ctx, cap, n + n / 4 + 16, p);
 }
+// a function's temporaries on the context's stream
+#define SOLVE_TMP(p, n)                                                                    \
+  do {                                                                                     \
+    if (!tmp.alloc(&(p), n)) return icf_fail(ctx, ICF_ERR_CUDA, "linear solve: out of memory"); \
+  } while (0)
 
 }  // namespace
 
@@ -918,10 +917,12 @@ static int build_order(icf_ctx *ctx) {
   unsigned *k0, *k1;
   int *i0;
   double *box;
-  ICF_CUDA(ctx, cudaMallocAsync(&k0, sizeof(unsigned) * (size_t)N, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&k1, sizeof(unsigned) * (size_t)N, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&i0, sizeof(int) * (size_t)N, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&box, sizeof(double) * 6, s));
+  icf_stream_mem mem{s};
+  icf_temps<icf_stream_mem> tmp(mem);
+  SOLVE_TMP(k0, N);
+  SOLVE_TMP(k1, N);
+  SOLVE_TMP(i0, N);
+  SOLVE_TMP(box, 6);
   k_bounds<<<1, 1024, 0, s>>>(n, ctx->d_x0, box);
   ICF_CUDA(ctx, cudaMemsetAsync(k0, 0xff, sizeof(unsigned) * (size_t)N, s));
   k_morton<<<icf_blocks(n, 256), 256, 0, s>>>(n, N, ctx->d_x0, ctx->d_alt, box, k0);
@@ -932,7 +933,6 @@ static int build_order(icf_ctx *ctx) {
   ICF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(ctx->d_tmp, tb, k0, k1, i0, S.perm, N, 0, 32, s));
   k_invert<<<icf_blocks(N, 256), 256, 0, s>>>(N, S.perm, S.iperm);
   ICF_CUDA(ctx, cudaGetLastError());
-  for (void *p : {(void *)k0, (void *)k1, (void *)i0, (void *)box}) ICF_CUDA(ctx, cudaFreeAsync(p, s));
   S.order_rows = N;
   return ICF_OK;
 }
@@ -954,20 +954,21 @@ static int build_steps(icf_ctx *ctx) {
   ICF_TRY_RC(grow(ctx, &S.ecol, &S.ecol_cap, 3 * scap));
   ICF_TRY_RC(grow(ctx, &S.eidx, &S.eidx_cap, 3 * scap));
   ICF_TRY_RC(grow(ctx, &S.last, &S.last_cap, scap));
-  if (!S.part) {  // the warps' first positions and batches, the halo counts, the maxima
-    ICF_CUDA(ctx, cudaMalloc(&S.part, sizeof(int) * ((2 * MR_WARPS + 1) * (size_t)ctx->n_sm + 8)));
-    ICF_CUDA(ctx, cudaMalloc(&S.hcol, sizeof(int) * (size_t)MR_HALO * ctx->n_sm));
-  }
+  // the warps' first positions and batches, the halo counts, the maxima
+  ICF_TRY_RC(grow(ctx, &S.part, &S.part_cap, (2 * MR_WARPS + 1) * (long long)ctx->n_sm + 8));
+  ICF_TRY_RC(grow(ctx, &S.hcol, &S.hcol_cap, (long long)MR_HALO * ctx->n_sm));
   S.first = S.part + MR_WARPS * ctx->n_sm + 1;
   S.hcount = S.first + MR_WARPS * ctx->n_sm + 1;
   int *d_most = S.hcount + ctx->n_sm;
   unsigned *k0, *k1;
   int *s0, *s1, *lrow, *steps, *raw;
-  ICF_CUDA(ctx, cudaMallocAsync(&k0, sizeof(unsigned) * (size_t)nnz, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&k1, sizeof(unsigned) * (size_t)nnz, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&s0, sizeof(int) * (size_t)nnz, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&s1, sizeof(int) * (size_t)nnz, s));
-  ICF_CUDA(ctx, cudaMallocAsync(&lrow, sizeof(int) * 3 * ((size_t)N + 1), s));
+  icf_stream_mem mem{s};
+  icf_temps<icf_stream_mem> tmp(mem);
+  SOLVE_TMP(k0, nnz);
+  SOLVE_TMP(k1, nnz);
+  SOLVE_TMP(s0, nnz);
+  SOLVE_TMP(s1, nnz);
+  SOLVE_TMP(lrow, 3 * (N + 1LL));
   steps = lrow + N + 1;
   raw = steps + N + 1;
   k_lower_keys<<<icf_blocks(nnz, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, k0, s0);
@@ -1001,7 +1002,6 @@ static int build_steps(icf_ctx *ctx) {
   int h[4] = {0, 0, 0, 0};
   ICF_CUDA(ctx, cudaMemcpyAsync(h, d_most, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
   ICF_CUDA(ctx, cudaMemcpyAsync(h + 3, S.first + nw, sizeof(int), cudaMemcpyDeviceToHost, s));
-  for (void *p : {(void *)k0, (void *)k1, (void *)s0, (void *)s1, (void *)lrow}) ICF_CUDA(ctx, cudaFreeAsync(p, s));
   ICF_CUDA(ctx, cudaStreamSynchronize(s));
   std::copy(h, h + 3, S.most);
   S.n_steps = MR_BATCH * (long long)h[3];

@@ -1,6 +1,7 @@
 """The growth of device arrays when allocations fail, over an allocator that
 fails where it is told to (compiled here with g++; no GPU): whatever fails, no
-capacity claims an array that is not there, and the next call makes up for it."""
+capacity claims an array that is not there, the next call makes up for it, and
+temporaries are returned."""
 import re
 import shutil
 import subprocess
@@ -34,6 +35,15 @@ struct fake {
 
 #define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); std::exit(1); } } while (0)
 
+static int temps(fake &m, int n) {
+  icf_temps<fake> t(m);
+  int *a;
+  double *b;
+  for (int i = 0; i < n; i++)
+    if (!(i % 2 ? t.alloc(&a, 10 + i) : t.alloc(&b, 3))) return 1;
+  return 0;
+}
+
 int main() {
   for (int fail = -1; fail < 3; fail++) {
     fake m;
@@ -59,6 +69,13 @@ int main() {
     int small_cap = 7;
     CHECK(icf_grow_all(m, &small_cap, 50, &a) && small_cap == 50);
   }
+  for (int n = 0; n <= 9; n++)
+    for (int fail = -1; fail < n; fail++) {
+      fake m;
+      m.fail_at = fail;
+      CHECK(temps(m, n) == (fail >= 0 || n > 8));
+      CHECK(m.live.empty());
+    }
   return 0;
 }
 """
@@ -74,9 +91,23 @@ def test_failed_allocations(tmp_path):
     assert out.returncode == 0, out.stdout
 
 
-def test_arrays_of_one_capacity_grow_together():
-    """The capacities of the structure's merge are set by the growth of their
-    arrays, never by hand."""
-    text = re.sub(r"//[^\n]*", "", (CSRC / "icf_pattern.cu").read_text())
-    caps = "rows_cap|items_cap|cols_cap|cr_cap|ks_cap|imp_pos_cap|s2m_cap|rhs_cap"
-    assert not re.findall(rf"\b(?:{caps})\s*=[^=]", text)
+CAPS = {"icf_pattern.cu": "rows_cap|items_cap|cols_cap|cr_cap|ks_cap|imp_pos_cap|s2m_cap|rhs_cap",
+        "icf_solve.cu": "[a-z]+_cap"}
+
+
+@pytest.mark.parametrize("name", sorted(CAPS))
+def test_arrays_of_one_capacity_grow_together(name):
+    """The capacities of the structure's merge and of the solver are set by the
+    growth of their arrays, never by hand."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    text = re.sub(r"\bhalo_cap\b", "", text)  # (a size, not a capacity)
+    assert not re.findall(rf"\b(?:{CAPS[name]})\s*=[^=]", text)
+
+
+def test_solver_allocates_by_capacity():
+    """No array of the solver hangs on whether another one is there, and its
+    temporaries are held by icf_temps."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "icf_solve.cu").read_text())
+    assert not re.findall(r"\bcuda(?:MallocAsync|FreeAsync)\b", text)
+    for m in re.finditer(r"cudaMalloc\(&(\S+?),", text):  # each under a check of its own
+        assert f"if (!{m.group(1)}) ICF_CUDA(ctx, cudaMalloc(&{m.group(1)}," in text, m.group(1)
