@@ -205,6 +205,7 @@ struct icf_solver {
   double *sc = nullptr, *h_sc = nullptr;  // scalars between launches, and pinned
   unsigned long long *slots = nullptr;    // the grid-wide exchanges' words
   unsigned epoch = 0;                     // exchanges numbered so far
+  int slice = 0;                          // iterations per launch if not the default (icf_solver_slice)
   int n_indefinite = 0;  // diagonal blocks of the last solve preconditioned by |S|^-1
 };
 

@@ -470,6 +470,7 @@ struct mr_args {
   double *sc;
   unsigned epoch0;  // number of the last exchange before this launch
   int max_iter, fresh;
+  int iters;        // iterations of this launch (a multiple of MR_CHECK)
   double tol;
 };
 
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(MR_THREADS, 1) k_minres(const mr_args A) {
   }
   __syncthreads();
   int status = S.status;
-  const int it_stop = it + MR_ITERS;
+  const int it_stop = it + A.iters;
   bool pending = false;  // the last iteration's w and x are still to be formed
   double *yin = A.y4, *yout = A.y4 + 4 * (size_t)A.N;
 
@@ -1011,6 +1012,15 @@ static int build_steps(icf_ctx *ctx) {
   return ICF_OK;
 }
 
+// Iterations per launch of this context's solves until its next static data: a
+// multiple of MR_CHECK up to 65,536, or 0 for MR_ITERS.  Not part of the
+// interface; for the tests of a solve that spans launches.
+extern "C" int icf_solver_slice(icf_ctx *ctx, int iters) {
+  if (!ctx || iters < 0 || iters > 65536 || iters % MR_CHECK != 0) return ICF_ERR_ARG;
+  ctx->solver.slice = iters;
+  return ICF_OK;
+}
+
 int icf_solve_impl(icf_ctx *ctx, double rel_tol, int max_iter, int *iters, double *relres) {
   icf_solver &S = ctx->solver;
   cudaStream_t s = ctx->stream;
@@ -1070,6 +1080,7 @@ int icf_solve_impl(icf_ctx *ctx, double rel_tol, int max_iter, int *iters, doubl
   A.slots = S.slots;
   A.sc = S.sc;
   A.max_iter = max_iter;
+  A.iters = S.slice > 0 ? S.slice : MR_ITERS;
   A.tol = rel_tol;
   A.fresh = 1;
   const void *fn = !halo                              ? (const void *)k_minres<false, 0, true>
@@ -1083,7 +1094,7 @@ int icf_solve_impl(icf_ctx *ctx, double rel_tol, int max_iter, int *iters, doubl
   const int *flags = reinterpret_cast<const int *>(S.h_sc + SC_BAD);
   do {
     A.epoch0 = S.epoch;
-    S.epoch += 2 * MR_ITERS + 2;
+    S.epoch += 2 * A.iters + 2;
     void *args[] = {&A};
     ICF_CUDA(ctx, cudaLaunchCooperativeKernel(fn, dim3(G), dim3(MR_THREADS), args, smem, s));
     ICF_CUDA(ctx, cudaMemcpyAsync(S.h_sc, S.sc, sizeof(double) * NSC, cudaMemcpyDeviceToHost, s));
