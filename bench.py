@@ -128,6 +128,7 @@ def kernel_share_bytes(name, nnz, n_rows, n_nodes, n_tet, n_cz, n_imp) -> int:
     algorithmic_bytes."""
     return {"k_tet_unit": 96 * n_nodes + 56 * n_tet,
             "k_cz_gp": 240 * n_cz,
+            "k_cz_lane": 240 * n_cz,
             "k_gather_off": 72 * (nnz - n_rows),
             "k_gather_diag": 72 * n_rows + 24 * n_rows,
             "k_gather_tile": 72 * nnz + 24 * n_rows,

@@ -961,20 +961,20 @@ constexpr int N_TET = 3;
 typedef void (*cz_fn)(int, const int *, const double4 *, const double *, const int *, const double4 *,
                       const double *, icf_dprm, icf_law_c, double *, double *, int *, double *, int *);
 struct cz_variant {
-  const char *name;
+  const char *name, *kernel;
   cz_fn f64, f32;
   int per_block, threads;
 };
-const cz_variant CZ_VARIANTS[] = {  // the first: or k_cz_lane, by cz_by_lane
-    {"96 thr, lane if large", k_cz_gp<false, 1>, k_cz_gp<true, 1>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
-    {"96 thr minb6", k_cz_gp<false, 6>, k_cz_gp<true, 6>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
-    {"96 thr minb8", k_cz_gp<false, 8>, k_cz_gp<true, 8>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
-    {"128 thr lane", k_cz_lane<false>, k_cz_lane<true>, CZ_LANES, CZ_LANES},
+const cz_variant CZ_VARIANTS[] = {
+    {"96 thr minb1", "k_cz_gp", k_cz_gp<false, 1>, k_cz_gp<true, 1>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
+    {"96 thr minb6", "k_cz_gp", k_cz_gp<false, 6>, k_cz_gp<true, 6>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
+    {"96 thr minb8", "k_cz_gp", k_cz_gp<false, 8>, k_cz_gp<true, 8>, CZ_PER_BLOCK, 3 * CZ_PER_BLOCK},
+    {"128 thr lane", "k_cz_lane", k_cz_lane<false>, k_cz_lane<true>, CZ_LANES, CZ_LANES},
 };
 // the kernel that settles every failure comparison with the reference's
 // rounding (the repeat of an assembly that left one undecided)
-const cz_variant CZ_EXACT = {"96 thr exact", k_cz_gp<false, 1, true>, k_cz_gp<true, 1, true>, CZ_PER_BLOCK,
-                              3 * CZ_PER_BLOCK};
+const cz_variant CZ_EXACT = {"96 thr exact", "k_cz_gp", k_cz_gp<false, 1, true>, k_cz_gp<true, 1, true>, CZ_PER_BLOCK,
+                             3 * CZ_PER_BLOCK};
 constexpr int N_CZV = sizeof(CZ_VARIANTS) / sizeof(CZ_VARIANTS[0]);
 
 int icf_tet_variants() { return N_TET; }
@@ -983,7 +983,7 @@ const char *icf_cz_variant_name(int v) { return CZ_VARIANTS[v].name; }
 
 static icf_law_c make_law_c(const icf_ctx *ctx, const icf_dprm &P);
 
-// k_cz_lane or k_cz_gp: by the time of their waves.  An SM holds 3 x 128 CZs of
+// Without a variant chosen, k_cz_lane or k_cz_gp: by the time of their waves.  An SM holds 3 x 128 CZs of
 // the one and (126 registers a thread) 5 x 32 of the other, and a lane evaluates
 // its three Gauss points in turn, so that a wave of k_cz_lane takes about twice
 // as long but has 2.4 times the CZs.  Below one wave of k_cz_gp, and where the
@@ -995,13 +995,17 @@ static bool cz_by_lane(const icf_ctx *ctx) {
   return 2 * ((ctx->n_cz + lane - 1) / lane) <= (ctx->n_cz + gp - 1) / gp;
 }
 
+static const cz_variant &cz_launched(const icf_ctx *ctx, int variant) {
+  if (ctx->cz_exact) return CZ_EXACT;
+  if (variant < 0 || variant >= N_CZV) variant = cz_by_lane(ctx) ? N_CZV - 1 : 0;
+  return CZ_VARIANTS[variant];
+}
+
 int icf_launch_cz(icf_ctx *ctx, int variant, const double4 *xc, double *cs, cudaStream_t s) {
   if (ctx->n_cz <= 0) return ICF_OK;
-  if (variant < 0 || variant >= N_CZV) variant = 0;
   const icf_dprm P = icf_make_dprm(ctx);
   const icf_law_c LC = make_law_c(ctx, P);
-  if (variant == 0 && cz_by_lane(ctx)) variant = N_CZV - 1;
-  const cz_variant &V = ctx->cz_exact ? CZ_EXACT : CZ_VARIANTS[variant];
+  const cz_variant &V = cz_launched(ctx, variant);
   const cz_fn f = ctx->precision == ICF_FP32_MIXED ? V.f32 : V.f64;
   f<<<icf_blocks(ctx->n_cz, V.per_block), V.threads, 0, s>>>(
       ctx->n_cz, ctx->d_cz, xc, ctx->d_czs, ctx->d_czfail, ctx->per_cz_prm ? ctx->d_czprm : nullptr, ctx->d_czhist,
@@ -1124,7 +1128,8 @@ static int enqueue_assembly(icf_ctx *ctx, double h) {
     ICF_TRY_RC(icf_launch_cz(ctx, ctx->tune_cz, ctx->d_xc, ctx->d_cs, scz));
     // ids, six node positions, state in, per-CZ strengths, staging, tentative
     // state, flags and averages out
-    icf_prof_mark(ctx, scz, "k_cz_gp", (24LL + 192 + 52 + (ctx->per_cz_prm ? 32 : 0) + cz_rec + 84) * ctx->n_cz);
+    icf_prof_mark(ctx, scz, cz_launched(ctx, ctx->tune_cz).kernel,
+                  (24LL + 192 + 52 + (ctx->per_cz_prm ? 32 : 0) + cz_rec + 84) * ctx->n_cz);
   }
   ICF_CUDA(ctx, cudaEventRecord(e_cz, sa));
 

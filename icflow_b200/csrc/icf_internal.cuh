@@ -405,7 +405,8 @@ struct icf_ctx {
   // on the main stream only and each kernel is followed by an event
   struct icf_prof_state *prof = nullptr;
   // launch variants chosen by the autotuner (indices into the variant tables)
-  int tune_tet = 0, tune_off = 0, tune_diag = 0, tune_cz = 0;
+  int tune_tet = 0, tune_off = 0, tune_diag = 0;
+  int tune_cz = -1;  // -1: by the model's size
   // staging layout of the tet contributions:
   //   ICF_LAYOUT_RECORDS  per-tet records es[8e + ...] read at random by the
   //                       gathers through the contribution codes;

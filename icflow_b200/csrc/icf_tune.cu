@@ -129,6 +129,7 @@ int icf_autotune_impl(icf_ctx *ctx, double h, int reps, icf_tune_report *out) {
       {"split", 5, ctx->n_cz > 0 ? 2 : 0, &split},
       {"streams", 7, 2, &serial},
       {"k_tet_unit", 0, ctx->n_elem > 0 ? icf_tet_variants() : 0, &ctx->tune_tet},
+      // (the name of the kind; k_cz_lane is one of its variants)
       {"k_cz_gp", 4, ctx->n_cz > 0 ? icf_cz_variants() : 0, &ctx->tune_cz},
       {"k_gather_off", 1, ctx->n_offd > 0 ? icf_gather_variants(0) : 0, &ctx->tune_off},
       {"k_gather_diag", 2, ctx->N > 0 ? icf_gather_variants(1) : 0, &ctx->tune_diag},
