@@ -197,6 +197,15 @@ struct row_cols {
   }
 };
 
+// Codes of a row that one warp sorts and places.  A list with a longer row (a
+// node or a face in hundreds of contacts) goes through k_item_* below as a whole:
+// the warp's network takes n log^2 n over 32 lanes, the radix sort of all codes
+// about 100 us more than a short list whatever the rows.  A call at 56,603 rows,
+// warp and whole list: 300 contacts of one face (1,200 codes a row) 400 and 265
+// us; 20,000 contacts, 80 to a face (320 codes) 258 and 328, 160 to a face 466 and
+// 369; 50,000 of one face 229 ms and 0.60 ms.
+constexpr int IMP_ROW_MAX = 512;
+
 struct int4_sum {
   __host__ __device__ int4 operator()(const int4 &a, const int4 &b) const {
     return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
@@ -215,13 +224,16 @@ __global__ void __launch_bounds__(256) k_imp_sort(int N, const int *__restrict__
                                                   unsigned long long *__restrict__ items,
                                                   const int *__restrict__ srow,
                                                   const unsigned long long *__restrict__ skey,
-                                                  int4 *__restrict__ stat) {
+                                                  int4 *__restrict__ stat, int *__restrict__ bad) {
   const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (r > N) return;
   const int b = r < N ? off[r] : 0, n = r < N ? off[r + 1] - b : 0;
   const int s0 = r < N ? srow[r] : 0, s1 = r < N ? srow[r + 1] : 0;
-  if (n == 0) {
-    if (lane == 0) stat[r] = make_int4(0, 0, 0, 0);
+  if (n == 0 || n > IMP_ROW_MAX) {
+    if (lane == 0) {
+      stat[r] = make_int4(0, 0, 0, 0);
+      if (n > 0) atomicOr(bad, 2);
+    }
     return;
   }
   unsigned long long *it = items + b;
@@ -335,6 +347,104 @@ __global__ void __launch_bounds__(256) k_imp_write(int N, int n_a, const int *__
     na += __popc(ma);
     no += __popc(mo);
   }
+}
+
+// ---- lists with long rows: one thread per code ------------------------------------
+// Every code with its key row << bits | column (bits: of the node count; all ones:
+// no code), in unit order, for a stable sort by key.
+__global__ void k_item_keys(int ni, const int4 *__restrict__ imp, const int *__restrict__ alt, int N,
+                            const int *__restrict__ diag, int bits, unsigned long long *__restrict__ key,
+                            unsigned *__restrict__ code, int *__restrict__ bad) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= ni) return;
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    key[16 * (size_t)u + k] = KMAX;
+    code[16 * (size_t)u + k] = (unsigned)u << 4 | (unsigned)k;
+  }
+  imp_codes(u, imp[u], alt, N, diag, bad, [&](int row, int col, unsigned c) {
+    key[c] = (unsigned long long)(unsigned)row << bits | (unsigned)col;
+  });
+}
+
+// place of a key's column among its row's static blocks, and whether it is one of them
+struct item_place {
+  int row, col, slot;  // slot: the first static block at or behind it
+  bool found;
+  __device__ __forceinline__ item_place(unsigned long long k, int bits, const int *__restrict__ srow,
+                                        const unsigned long long *__restrict__ skey) {
+    row = (int)(k >> bits);
+    col = (int)(k & ((1ull << bits) - 1));
+    const int s0 = srow[row], n = srow[row + 1] - s0;
+    const unsigned long long want = (unsigned long long)(unsigned)row << 32 | (unsigned)col;
+    const int p = lower_of(skey + s0, n, want);
+    slot = s0 + p;
+    found = p < n && skey[slot] == want;
+  }
+};
+
+// statistics of the code at i as k_imp_sort gives them for a row (i = n: zero,
+// for the scan), and its place in the list of codes
+__global__ void k_item_class(int n, int bits, const unsigned long long *__restrict__ key,
+                             const unsigned *__restrict__ code, const int *__restrict__ srow,
+                             const unsigned long long *__restrict__ skey, int4 *__restrict__ stat,
+                             int *__restrict__ pos) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > n) return;
+  int4 st = make_int4(0, 0, 0, 0);
+  if (i < n && key[i] != KMAX) {
+    pos[code[i]] = i;
+    if (i == 0 || key[i - 1] != key[i]) {
+      const item_place P(key[i], bits, srow, skey);
+      const bool diag = P.col == P.row;
+      st = make_int4(!P.found, !P.found || diag, P.found && !diag, 0);
+    }
+  }
+  stat[i] = st;
+}
+
+// the rows' prefix sums, as the scan of k_imp_sort's statistics gives them
+__global__ void k_item_rows(int N, const int *__restrict__ off, const int4 *__restrict__ ipre,
+                            int4 *__restrict__ pre) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r <= N) pre[r] = ipre[off[r]];
+}
+
+// what k_imp_write writes, by the first code of each block; the thread behind a
+// block's last code closes its record range
+__global__ void k_item_write(int n, int n_a, int bits, const unsigned long long *__restrict__ key,
+                             const int *__restrict__ srow, const unsigned long long *__restrict__ skey,
+                             const int4 *__restrict__ ipre, unsigned long long *__restrict__ mkey,
+                             int *__restrict__ cols, int *__restrict__ newcol, int2 *__restrict__ range,
+                             int *__restrict__ pslot, int *__restrict__ prow) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > n) return;
+  const unsigned long long k = i < n ? key[i] : KMAX, before = i > 0 ? key[i - 1] : KMAX;
+  if (k == before) return;
+  const int4 o = ipre[i];
+  if (before != KMAX) {
+    const item_place P(before, bits, srow, skey);
+    range[!P.found || P.col == P.row ? o.y - 1 : n_a + o.z - 1].y = i;
+  }
+  if (k == KMAX) return;
+  const item_place P(k, bits, srow, skey);
+  const bool diag = P.col == P.row;
+  const int w = !P.found || diag ? o.y : n_a + o.z, slot = P.slot + o.x;
+  range[w].x = i;
+  pslot[w] = slot;
+  prow[w] = diag ? P.row : (P.found ? -1 : -2);
+  if (!P.found) {
+    newcol[o.x] = P.col;
+    mkey[slot] = (unsigned long long)(unsigned)P.row << 32 | (unsigned)P.col;
+    cols[slot] = P.col;
+  }
+}
+
+// row starts of the merged pattern
+__global__ void k_item_starts(int N, const int *__restrict__ srow, const int4 *__restrict__ pre,
+                              int *__restrict__ rows) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r <= N) rows[r] = srow[r] + pre[r].x;
 }
 
 // the static blocks' merged positions: behind the new blocks of the rows
@@ -891,11 +1001,48 @@ void icf_free_dyn_ws(icf_ctx *ctx) {
   D = icf_dyn_ws();
 }
 
+// The codes of a list with long rows, sorted by row and column: their keys, and
+// for each the prefix sums of the statistics before it.
+struct sorted_items {
+  int bits = 0;
+  unsigned long long *key = nullptr;
+  int4 *pre = nullptr;
+};
+static int sort_items(icf_ctx *ctx, icf_temps<icf_stream_mem> &tmp, sorted_items &I) {
+  cudaStream_t s = ctx->stream;
+  icf_dyn_ws &D = ctx->dyn;
+  const int N = ctx->N, ni = ctx->n_imp, n = 16 * ni;
+  unsigned long long *k0, *k1;
+  unsigned *c0, *c1;
+  int4 *stat, *pre;
+  if (!tmp.alloc(&k0, n) || !tmp.alloc(&k1, n) || !tmp.alloc(&c0, n) || !tmp.alloc(&c1, n) ||
+      !tmp.alloc(&stat, n + 1LL) || !tmp.alloc(&pre, n + 1LL))
+    return icf_fail(ctx, ICF_ERR_CUDA, "contact structure: out of memory");
+  int bits = 1;
+  while ((1LL << bits) <= (long long)ctx->n_nodes) bits++;  // (rows and columns are below, so no key has all bits set)
+  k_item_keys<<<icf_blocks(ni, 128), 128, 0, s>>>(ni, ctx->d_imp, ctx->d_alt, N, ctx->d_diag, bits, k0, c0, D.small);
+  size_t tb = 0, tb2 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tb, k0, k1, c0, c1, n, 0, 2 * bits, s);
+  cub::DeviceScan::ExclusiveScan(nullptr, tb2, stat, pre, int4_sum(), make_int4(0, 0, 0, 0), n + 1, s);
+  if (icf_scratch(ctx, tb > tb2 ? tb : tb2)) return ICF_ERR_CUDA;
+  ICF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(ctx->d_tmp, tb, k0, k1, c0, c1, n, 0, 2 * bits, s));
+  k_item_class<<<icf_blocks(n + 1LL, 256), 256, 0, s>>>(n, bits, k1, c1, ctx->d_srow, ctx->d_skeys, stat,
+                                                      ctx->d_imp_pos);
+  ICF_CUDA(ctx, cub::DeviceScan::ExclusiveScan(ctx->d_tmp, tb2, stat, pre, int4_sum(), make_int4(0, 0, 0, 0), n + 1, s));
+  k_item_rows<<<icf_blocks(N + 1LL, 256), 256, 0, s>>>(N, D.off, pre, D.pre);
+  ICF_CUDA(ctx, cudaGetLastError());
+  I = {bits, k1, pre};
+  return ICF_OK;
+}
+
 int icf_build_merged_pattern(icf_ctx *ctx) {
   cudaStream_t s = ctx->stream;
   const int nnz_s = ctx->nnz_s, N = ctx->N, ni = ctx->n_imp;
   icf_dyn_ws &D = ctx->dyn;
   int4 tot = make_int4(0, 0, 0, 0);  // new blocks; touched ones of each part
+  icf_stream_mem mem{s};
+  icf_temps<icf_stream_mem> tmp(mem);
+  sorted_items I;
   if (ni > 0) {
     // per-row work arrays (cnt stays zero between builds) and the items
     if (N + 1 > D.rows_cap) {
@@ -916,14 +1063,20 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
     ICF_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->d_tmp, tb, D.cnt, D.off, N + 1, s));
     k_imp_place<<<icf_blocks(ni, 128), 128, 0, s>>>(ni, ctx->d_imp, ctx->d_alt, N, ctx->d_diag, D.off, D.cnt, D.items,
                                                    D.small);
-    k_imp_sort<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, D.off, D.items, ctx->d_srow, ctx->d_skeys, D.stat);
+    k_imp_sort<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, D.off, D.items, ctx->d_srow, ctx->d_skeys, D.stat,
+                                                             D.small);
     ICF_CUDA(ctx, cub::DeviceScan::ExclusiveScan(ctx->d_tmp, tb2, D.stat, D.pre, int4_sum(), make_int4(0, 0, 0, 0),
                                                  N + 1, s));
     ICF_CUDA(ctx, cudaGetLastError());
     ICF_CUDA(ctx, cudaMemcpyAsync(D.h_small, D.pre + N, sizeof(int4), cudaMemcpyDeviceToHost, s));
     ICF_CUDA(ctx, cudaMemcpyAsync(D.h_small + 4, D.small, sizeof(int), cudaMemcpyDeviceToHost, s));
     ICF_CUDA(ctx, cudaStreamSynchronize(s));
-    if (D.h_small[4]) return icf_fail(ctx, ICF_ERR_STATE, "an impact references a row outside the pattern");
+    if (D.h_small[4] & 1) return icf_fail(ctx, ICF_ERR_STATE, "an impact references a row outside the pattern");
+    if (D.h_small[4] & 2) {
+      ICF_TRY_RC(sort_items(ctx, tmp, I));
+      ICF_CUDA(ctx, cudaMemcpyAsync(D.h_small, D.pre + N, sizeof(int4), cudaMemcpyDeviceToHost, s));
+      ICF_CUDA(ctx, cudaStreamSynchronize(s));
+    }
     tot = make_int4(D.h_small[0], D.h_small[1], D.h_small[2], 0);
   }
   const int nd = tot.x, nnz = nnz_s + nd;
@@ -941,10 +1094,18 @@ int icf_build_merged_pattern(icf_ctx *ctx) {
     if (n_crs + 1 > ctx->cr_cap)
       ICF_TRY_RC(icf_grow(ctx, &ctx->cr_cap, n_crs + n_crs / 4 + 16LL, &ctx->d_cr_range, &ctx->d_cr_pslot,
                           &ctx->d_cr_row));
-    k_imp_write<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, tot.y, D.off, D.items, ctx->d_srow, ctx->d_skeys,
-                                                              D.pre, ctx->d_rows, ctx->d_mkeys, ctx->d_cols, D.newcol,
-                                                              ctx->d_imp_pos, ctx->d_cr_range, ctx->d_cr_pslot,
-                                                              ctx->d_cr_row);
+    if (I.key) {
+      k_item_starts<<<icf_blocks(N + 1LL, 256), 256, 0, s>>>(N, ctx->d_srow, D.pre, ctx->d_rows);
+      k_item_write<<<icf_blocks(16LL * ni + 1, 256), 256, 0, s>>>(16 * ni, tot.y, I.bits, I.key, ctx->d_srow,
+                                                                ctx->d_skeys, I.pre, ctx->d_mkeys, ctx->d_cols,
+                                                                D.newcol, ctx->d_cr_range, ctx->d_cr_pslot,
+                                                                ctx->d_cr_row);
+    } else {
+      k_imp_write<<<icf_blocks(32 * (N + 1LL), 256), 256, 0, s>>>(N, tot.y, D.off, D.items, ctx->d_srow, ctx->d_skeys,
+                                                                D.pre, ctx->d_rows, ctx->d_mkeys, ctx->d_cols,
+                                                                D.newcol, ctx->d_imp_pos, ctx->d_cr_range,
+                                                                ctx->d_cr_pslot, ctx->d_cr_row);
+    }
     if (nnz_s > 0)
       k_merge_static<<<icf_blocks(nnz_s, 256), 256, 0, s>>>(nnz_s, ctx->d_skeys, D.pre, D.newcol, ctx->d_mkeys,
                                                            ctx->d_cols, ctx->d_s2m);
