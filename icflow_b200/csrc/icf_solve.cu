@@ -98,14 +98,17 @@ __global__ void k_invert(int n, const int *__restrict__ perm, int *__restrict__ 
   if (i < n) iperm[perm[i]] = i;
 }
 
-// sort key of slot s: its column, N for a diagonal block (after every column)
+// sort key of slot s: its column, N for a diagonal block (after every column) and
+// for a column without a row (a contact with a node that no unit holds), which
+// sets *outside
 __global__ void k_lower_keys(int N, int nnz, const unsigned long long *__restrict__ mkeys, unsigned *__restrict__ key,
-                             int *__restrict__ slot) {
+                             int *__restrict__ slot, int *__restrict__ outside) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nnz) return;
   const unsigned long long k = mkeys[s];
   const unsigned r = (unsigned)(k >> 32), c = (unsigned)(k & 0xffffffffull);
-  key[s] = r == c ? (unsigned)N : c;
+  key[s] = r == c || c >= (unsigned)N ? (unsigned)N : c;
+  if (c >= (unsigned)N) *outside = 1;
   slot[s] = s;
 }
 
@@ -149,7 +152,7 @@ __global__ void k_entries(int N, int nnz, const unsigned long long *__restrict__
     const int r = (int)(k >> 32), p = iperm[r], i = q - rows[r];
     const int e = 3 * sstep[p] + i;
     eslot[e] = (int)((unsigned)q << 1);
-    ecol[e] = iperm[(int)(k & 0xffffffffull)];
+    ecol[e] = iperm[min((int)(k & 0xffffffffull), N - 1)];
   }
   const unsigned c = key[q];
   if (c < (unsigned)N) {
@@ -955,7 +958,7 @@ static int build_steps(icf_ctx *ctx) {
   ICF_TRY_RC(grow(ctx, &S.ecol, &S.ecol_cap, 3 * scap));
   ICF_TRY_RC(grow(ctx, &S.eidx, &S.eidx_cap, 3 * scap));
   ICF_TRY_RC(grow(ctx, &S.last, &S.last_cap, scap));
-  // the warps' first positions and batches, the halo counts, the maxima
+  // the warps' first positions and batches, the halo counts, the maxima and a flag
   ICF_TRY_RC(grow(ctx, &S.part, &S.part_cap, (2 * MR_WARPS + 1) * (long long)ctx->n_sm + 8));
   ICF_TRY_RC(grow(ctx, &S.hcol, &S.hcol_cap, (long long)MR_HALO * ctx->n_sm));
   S.first = S.part + MR_WARPS * ctx->n_sm + 1;
@@ -972,7 +975,8 @@ static int build_steps(icf_ctx *ctx) {
   SOLVE_TMP(lrow, 3 * (N + 1LL));
   steps = lrow + N + 1;
   raw = steps + N + 1;
-  k_lower_keys<<<icf_blocks(nnz, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, k0, s0);
+  ICF_CUDA(ctx, cudaMemsetAsync(d_most, 0, 4 * sizeof(int), s));
+  k_lower_keys<<<icf_blocks(nnz, 256), 256, 0, s>>>(N, nnz, ctx->d_mkeys, k0, s0, d_most + 3);
   int bits = 1;
   while ((1LL << bits) <= (long long)N) bits++;
   size_t tb = 0, tb2 = 0;
@@ -983,7 +987,6 @@ static int build_steps(icf_ctx *ctx) {
   k_lower_rows<<<icf_blocks(N + 1LL, 256), 256, 0, s>>>(N, nnz, k1, lrow);
   k_steps<<<icf_blocks(N + 1LL, 256), 256, 0, s>>>(N, S.perm, ctx->d_rows, lrow, steps);
   ICF_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->d_tmp, tb2, steps, raw, N + 1, s));
-  ICF_CUDA(ctx, cudaMemsetAsync(d_most, 0, 3 * sizeof(int), s));
   k_part<<<icf_blocks(nw + 1LL, 128), 128, 0, s>>>(N, nw, raw, S.part, S.first, d_most);
   k_first<<<1, 1024, 0, s>>>(nw, S.first);
   ICF_CUDA(ctx, cudaMemsetAsync(S.eslot, 0xff, sizeof(int) * 3 * (size_t)scap, s));
@@ -1000,12 +1003,13 @@ static int build_steps(icf_ctx *ctx) {
     k_halo<<<G, 512, hsm, s>>>(N, S.first, S.eslot, S.ecol, S.hcol, S.hcount, S.eidx, d_most);
   }
   ICF_CUDA(ctx, cudaGetLastError());
-  int h[4] = {0, 0, 0, 0};
-  ICF_CUDA(ctx, cudaMemcpyAsync(h, d_most, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  ICF_CUDA(ctx, cudaMemcpyAsync(h + 3, S.first + nw, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int h[5] = {0, 0, 0, 0, 0};
+  ICF_CUDA(ctx, cudaMemcpyAsync(h, d_most, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  ICF_CUDA(ctx, cudaMemcpyAsync(h + 4, S.first + nw, sizeof(int), cudaMemcpyDeviceToHost, s));
   ICF_CUDA(ctx, cudaStreamSynchronize(s));
+  if (h[3]) return icf_fail(ctx, ICF_ERR_STATE, "linear solve: a contact joins a row to a node outside the system");
   std::copy(h, h + 3, S.most);
-  S.n_steps = MR_BATCH * (long long)h[3];
+  S.n_steps = MR_BATCH * (long long)h[4];
   S.blocks = G;
   S.halo = try_halo && h[1] <= MR_HALO;
   S.gen = ctx->struct_gen;
