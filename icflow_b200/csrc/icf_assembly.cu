@@ -757,12 +757,12 @@ __global__ void k_infer(int n, double h, double beta, double gamma,
   va[3 * i + 2] = make_double2(anx[1], anx[2]);
 }
 
-__global__ void k_add_dx(int n, const int *__restrict__ alt,
+__global__ void k_add_dx(int n, int N, const int *__restrict__ alt,
                          const double *__restrict__ dx, double *__restrict__ du) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int r = alt[i];
-  if (r < 0) return;
+  if (r < 0 || r >= N) return;  // (past the last row: a node that no unit holds)
   for (int k = 0; k < 3; k++) du[3 * (size_t)i + k] += dx[3 * (size_t)r + k];
 }
 
@@ -1389,7 +1389,7 @@ int icf_launch_infer(icf_ctx *ctx, double h) {
 }
 
 int icf_launch_add_dx(icf_ctx *ctx, const double *d_dx) {
-  k_add_dx<<<icf_blocks(ctx->n_nodes, 256), 256, 0, ctx->stream>>>(ctx->n_nodes, ctx->d_alt, d_dx,
+  k_add_dx<<<icf_blocks(ctx->n_nodes, 256), 256, 0, ctx->stream>>>(ctx->n_nodes, ctx->N, ctx->d_alt, d_dx,
                                                                   ctx->d_du);
   const int n = 3 * ctx->N;
   const int nb = 256;
