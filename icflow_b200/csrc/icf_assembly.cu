@@ -599,7 +599,7 @@ __device__ __forceinline__ void add_row3(double *o, const double v[3]) {
 // two loads) are summed in FP64, in code order, and added to the block, and to
 // the rhs row for a diagonal block (row >= 0).  A block that only contact
 // pairs create (row == -2) is written, not added to: nothing else writes it.
-// The touched blocks come in k_imp_add's order (icf_pattern.cu k_split_off):
+// The touched blocks come in k_imp_add's order (icf_pattern.cu k_imp_write):
 // the launch over [first, first + count) reads its metadata contiguously.
 __device__ __forceinline__ double4 ld_nc4(const double4 *p) {
   double4 r;
@@ -1212,8 +1212,8 @@ static int enqueue_assembly(icf_ctx *ctx, double h) {
   ICF_CUDA(ctx, cudaEventRecord(e_a, sa));
   ICF_CUDA(ctx, cudaEventRecord(e_b, sb));
   // impact terms: the blocks that the off-diagonal gather does not write
-  // (diagonal blocks, written on main, and contact-only blocks, zeroed on
-  // aux1) as soon as the impacts are staged; the others after the join
+  // (diagonal blocks, written on main, and contact-only blocks, which these
+  // launches write) as soon as the impacts are staged; the others after the join
   // algorithmic bytes: the impact staging once, 172 B per touched block and
   // 4 B per code, split between the two launches by their blocks
   const long long n_codes = 10LL * ctx->n_imp;  // at most; records of 12 doubles

@@ -17,7 +17,7 @@
 //             ks[ni*132] double                   per impact: the records of its
 //                                                 codes (<= 10 x 12) + 12 forces
 //   pattern   static keys (row<<32|col) sorted, rc_off[nnz_s+1], rc[] codes
-//             merged pattern rows/cols + src (static index of merged slot)
+//             merged pattern rows/cols, s2m (merged slot of a static slot)
 //
 // Contribution codes (32 bit), one per (unit, row vertex a, column vertex b)
 // with alt(b) >= alt(a):

@@ -255,7 +255,6 @@ struct grad_smem {
   float W2[NH * NH];  // the bf16 values
   float W3[NO * NH];
   float B1[NH], B2[NH], B3[NO + 1];
-  float norm[2 * NI + 2];
   float x[NODES][16];                    // normalised, rounded to bf16; column 15 zero
   float z1[NODES][LDH], z2[NODES][LDH];  // pre-activations, later dZ1 and dZ2
   float h1[NODES][LDH], h2[NODES][LDH];  // bf16 values

@@ -17,8 +17,9 @@
 //
 // All calls on a device share the one array and it keeps the contents of the
 // last call; everything a call reads from it is written earlier in the same
-// call, and the counters that must start at zero live in the context and are
-// cleared on the stream first.  Calls whose work overlaps on the GPU (two
+// call, and the counters that must start at zero live in the context, where
+// every assembly leaves zeros behind (a call after one that failed clears them
+// on the stream first).  Calls whose work overlaps on the GPU (two
 // threads, two contexts on one device, or two streams) race on the array; the
 // entry point is synchronous, so calls made one after another from one thread
 // do not overlap.

@@ -20,7 +20,8 @@
 // blocks.  (A 64-bit radix sort of 16 keys per impact, another of the codes by
 // slot, run-length encodings and six synchronisations took 410 us of kernels
 // and as much again of allocations and waiting at 22,687 impacts, 490 us a call;
-// this takes 100 us of kernels and 138 us a call, one synchronisation among it.)
+// this takes 100 us of kernels and 138 us a call, with two synchronisations: the
+// sizes, and the end of the call.)  Only a list with long rows is sorted as a whole.
 #include <cub/cub.cuh>
 
 #include "icf_internal.cuh"

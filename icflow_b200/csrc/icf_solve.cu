@@ -166,8 +166,12 @@ __global__ void k_entries(int N, int nnz, const unsigned long long *__restrict__
 // (a row weighs its steps and MR_ROW_WEIGHT more for its vectors).  A warp's
 // steps start at a multiple of MR_BATCH: first[w], the number of batches before
 // it (turned into a prefix sum by k_first).  most[0]: the largest thread block's
-// rows, most[2]: the largest warp's batches.
-constexpr int MR_ROW_WEIGHT = 5;  // (0 to 6 measured alike)
+// rows, most[2]: the largest warp's batches.  Row weights of 0 to 6, and 16 to 48
+// rows a block at least (MR_MIN_ROWS), take the same time.  They decide the order
+// of the sums, though, and with it the last digits that the Newton runs of the
+// tests carry through contact events: these are the values those runs were
+// checked with.
+constexpr int MR_ROW_WEIGHT = 5;
 constexpr int MR_WARPS = 16;  // of a thread block of k_minres
 constexpr int MR_BATCH = 8;   // steps a warp reads together
 __device__ int first_at(const int *__restrict__ raw, int lo, int hi, long long target) {
@@ -451,7 +455,7 @@ __device__ void precond_row(const double *__restrict__ a, double *o, int *bad) {
 // orders nothing in memory and needs no fence.  A wait that runs out of polls
 // sets the status and every block returns.
 constexpr int MR_THREADS = 32 * MR_WARPS;
-constexpr int MR_MIN_ROWS = 24;          // a block is given at least so many rows (16 to 48 measured alike)
+constexpr int MR_MIN_ROWS = 24;          // a block is given at least so many rows (see k_part)
 constexpr int MR_CAP = 10;               // rows a warp adds up together
 constexpr int MR_ITERS = 2048;           // iterations per launch (a multiple of MR_CHECK)
 constexpr int MR_CHECK = 4;              // the stopping test, every so many iterations
