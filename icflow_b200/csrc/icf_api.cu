@@ -704,11 +704,9 @@ int icf_narrow_phase(icf_ctx *ctx, int n_pairs, const int *pairs, int *n_impacts
   if (ctx->n_surf == 0) return icf_fail(ctx, ICF_ERR_STATE, "no surface elements were transferred");
   for (long long i = 0; i < 2LL * n_pairs; i++)
     if (pairs[i] < 0 || pairs[i] >= ctx->n_surf) return icf_fail(ctx, ICF_ERR_ARG, "pair element id out of range");
-  if (n_pairs > ctx->pairs_cap) {
-    ICF_TRY(dalloc(ctx, &ctx->d_pairs, 2 * (size_t)n_pairs));
-    ICF_TRY(dalloc(ctx, &ctx->d_masks, (size_t)n_pairs));
-    ctx->pairs_cap = n_pairs;
-  }
+  if (n_pairs > ctx->pairs_cap)
+    ICF_TRY(icf_grow(ctx, &ctx->pairs_cap, n_pairs, icf_of(&ctx->d_pairs, 2LL * n_pairs),
+                     icf_of(&ctx->d_masks, n_pairs)));
   ICF_CUDA(ctx, cudaMemcpyAsync(ctx->d_pairs, pairs, sizeof(int) * 2 * (size_t)n_pairs, cudaMemcpyHostToDevice,
                                 ctx->stream));
   ctx->n_pairs = n_pairs;
@@ -741,9 +739,8 @@ int icf_set_impacts(icf_ctx *ctx, int n_impacts, const int *impacts) {
   for (long long i = 0; i < 4LL * n_impacts; i++)
     if (impacts[i] < 0 || impacts[i] >= ctx->n_nodes) return icf_fail(ctx, ICF_ERR_ARG, "impact node id out of range");
   if (n_impacts > ctx->imp_cap) {
-    ICF_TRY(dalloc(ctx, &ctx->d_imp, 2 * (size_t)n_impacts));
-    ctx->imp_cap = 2 * n_impacts;
     ctx->imp_gen++;
+    ICF_TRY(icf_grow(ctx, &ctx->imp_cap, 2LL * n_impacts, &ctx->d_imp));
   }
   if (n_impacts)
     ICF_CUDA(ctx, icf_h2d(ctx->stream, ctx->d_imp, impacts, sizeof(int4) * (size_t)n_impacts));
@@ -805,12 +802,8 @@ int icf_create_structure(icf_ctx *ctx, int *N, int *nnz) {
   ICF_TRY(icf_build_merged_pattern(ctx));
   if (ctx->gather_tiles && !ctx->tiles.built) ICF_TRY(icf_build_tiles(ctx));
   // remember the impacts this structure holds
-  if (ctx->n_imp > ctx->imp_built_cap) {
-    cudaFree(ctx->d_imp_built);
-    ctx->d_imp_built = nullptr;
-    ICF_TRY(dalloc(ctx, &ctx->d_imp_built, 2 * (size_t)ctx->n_imp));
-    ctx->imp_built_cap = 2 * ctx->n_imp;
-  }
+  if (ctx->n_imp > ctx->imp_built_cap)
+    ICF_TRY(icf_grow(ctx, &ctx->imp_built_cap, 2LL * ctx->n_imp, &ctx->d_imp_built));
   if (ctx->n_imp)
     ICF_CUDA(ctx, cudaMemcpyAsync(ctx->d_imp_built, ctx->d_imp, sizeof(int4) * (size_t)ctx->n_imp,
                                   cudaMemcpyDeviceToDevice, ctx->stream));

@@ -558,12 +558,8 @@ int icf_broad_phase_impl(icf_ctx *ctx, double pad, const int *d_group, int *n_pa
   ICF_TRY_RC(ensure_small(ctx));
   const int nbk = (int)std::min<long long>((n + 255) / 256, 2LL * ctx->n_sm);
   if (n > W.b_cap) {
-    ICF_TRY_RC(grow(ctx, &W.lohi, 6LL * n));
-    ICF_TRY_RC(grow(ctx, &W.ext, n));
-    ICF_TRY_RC(grow(ctx, &W.bcnt, n + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.boff, n + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.clo, n));
-    W.b_cap = n;
+    ICF_TRY_RC(icf_grow(ctx, &W.b_cap, n, icf_of(&W.lohi, 6LL * n), icf_of(&W.ext, n), icf_of(&W.bcnt, n + 1LL),
+                        icf_of(&W.boff, n + 1LL), icf_of(&W.clo, n)));
   }
   if (!W.tmpv) ICF_TRY_RC(grow(ctx, &W.tmpv, 8LL * (2 * ctx->n_sm + 1)));
   if (!W.red) ICF_TRY_RC(grow(ctx, &W.red, 8));
@@ -598,13 +594,8 @@ int icf_broad_phase_impl(icf_ctx *ctx, double pad, const int *d_group, int *n_pa
   while ((1LL << pb) < (long long)n) pb++;
   if (m > W.ent_cap) {
     const long long c = m + m / 4 + 64;
-    ICF_TRY_RC(grow(ctx, &W.ek0, c));
-    ICF_TRY_RC(grow(ctx, &W.ek1, c));
-    ICF_TRY_RC(grow(ctx, &W.ee0, c));
-    ICF_TRY_RC(grow(ctx, &W.ee1, c));
-    ICF_TRY_RC(grow(ctx, &W.pc, c + 1));
-    ICF_TRY_RC(grow(ctx, &W.po, c + 1));
-    W.ent_cap = c;
+    ICF_TRY_RC(icf_grow(ctx, &W.ent_cap, c, icf_of(&W.ek0, c), icf_of(&W.ek1, c), icf_of(&W.ee0, c),
+                        icf_of(&W.ee1, c), icf_of(&W.pc, c + 1), icf_of(&W.po, c + 1)));
   }
   k_entries<<<icf_blocks(n, 256), 256, 0, s>>>(n, W.clo, W.boff, nb, gbits, d_group, W.ek0, W.ee0);
   const int end_bit = gbits >= 0 ? 3 * nb + gbits : 3 * nb;
@@ -622,19 +613,11 @@ int icf_broad_phase_impl(icf_ctx *ctx, double pad, const int *d_group, int *n_pa
   for (int attempt = 0; attempt < 2; attempt++) {
     if (W.pair_cap == 0) {
       const long long c = std::max<long long>(4LL * n, 1024);
-      ICF_TRY_RC(grow(ctx, &W.p0, c));
-      ICF_TRY_RC(grow(ctx, &W.p1, c));
-      W.pair_cap = c;
+      ICF_TRY_RC(icf_grow(ctx, &W.pair_cap, c, &W.p0, &W.p1));
     }
     const long long P = W.pair_cap;
-    if (P > ctx->pairs_cap || !ctx->d_pairs) {
-      cudaFree(ctx->d_pairs);
-      cudaFree(ctx->d_masks);
-      ctx->d_pairs = ctx->d_masks = nullptr;
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_pairs, sizeof(int) * 2 * (size_t)P));
-      ICF_CUDA(ctx, cudaMalloc(&ctx->d_masks, sizeof(int) * (size_t)P));
-      ctx->pairs_cap = (int)P;
-    }
+    if (P > ctx->pairs_cap)
+      ICF_TRY_RC(icf_grow(ctx, &ctx->pairs_cap, P, icf_of(&ctx->d_pairs, 2 * P), icf_of(&ctx->d_masks, P)));
     // pad with all-ones keys: they sort after every pair and form one run
     ICF_CUDA(ctx, cudaMemsetAsync(W.p0, 0xFF, sizeof(unsigned long long) * (size_t)P, s));
     k_pairs<<<icf_blocks(m, 128), 128, 0, s>>>(m, W.ek1, W.ee1, W.lohi, W.clo, nb, d_group, gbits, ctx->d_selem, ctx->d_xc,
@@ -658,9 +641,7 @@ int icf_broad_phase_impl(icf_ctx *ctx, double pad, const int *d_group, int *n_pa
     }
     // more candidate pairs than the buffer holds: grow it and write them again
     const long long c = nall + nall / 4 + 1024;
-    ICF_TRY_RC(grow(ctx, &W.p0, c));
-    ICF_TRY_RC(grow(ctx, &W.p1, c));
-    W.pair_cap = c;
+    ICF_TRY_RC(icf_grow(ctx, &W.pair_cap, c, &W.p0, &W.p1));
   }
   return icf_fail(ctx, ICF_ERR_SIZE, "broad phase: pair buffer growth did not converge");
 }
@@ -777,19 +758,14 @@ static int detect_pass(icf_ctx *ctx, double pad, const int *d_group, int *n_impa
   if (st == 2) return icf_fail(ctx, ICF_ERR_SIZE, "contact detection: grid too large");
   if (st == 3) {  // more cells than the buffers hold
     const long long c = W.h_gp[3] + W.h_gp[3] / 4 + 2;
-    ICF_TRY_RC(grow(ctx, &W.gcnt, c));
-    ICF_TRY_RC(grow(ctx, &W.goff, c));
-    ICF_TRY_RC(grow(ctx, &W.gcur, c));
+    ICF_TRY_RC(icf_grow(ctx, &W.cell_cap, c, &W.gcnt, &W.goff, &W.gcur));
     ICF_CUDA(ctx, cudaMemsetAsync(W.gcnt, 0, sizeof(int) * (size_t)c, s));
-    W.cell_cap = c;
     *again = true;
   }
   const long long hits = W.h_small[2];  // candidates, before the pair rule
   if (hits > W.nkey_cap) {  // more candidates than the key buffers hold
     const long long c = hits + hits / 4 + 1024;
-    ICF_TRY_RC(grow(ctx, &W.nk0, c));
-    ICF_TRY_RC(grow(ctx, &W.nk1, c));
-    W.nkey_cap = c;
+    ICF_TRY_RC(icf_grow(ctx, &W.nkey_cap, c, &W.nk0, &W.nk1));
     *again = true;
   }
   return ICF_OK;
@@ -808,26 +784,17 @@ int icf_detect_contacts_impl(icf_ctx *ctx, double pad, const int *d_group, int *
     return icf_fail(ctx, ICF_ERR_SIZE, "contact detection: more than 2^26 nodes");
   ICF_TRY_RC(ensure_small(ctx));
   if (n > W.b_cap) {
-    ICF_TRY_RC(grow(ctx, &W.lohi, 6LL * n));
-    ICF_TRY_RC(grow(ctx, &W.ext, n));
-    ICF_TRY_RC(grow(ctx, &W.bcnt, n + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.boff, n + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.clo, n));
-    W.b_cap = n;
+    ICF_TRY_RC(icf_grow(ctx, &W.b_cap, n, icf_of(&W.lohi, 6LL * n), icf_of(&W.ext, n), icf_of(&W.bcnt, n + 1LL),
+                        icf_of(&W.boff, n + 1LL), icf_of(&W.clo, n)));
   }
   if (ns > W.gnode_cap) {
-    ICF_TRY_RC(grow(ctx, &W.gnode, ns));
-    W.gnode_cap = ns;
+    ICF_TRY_RC(icf_grow(ctx, &W.gnode_cap, ns, &W.gnode));
   }
   if (n > W.tinv_cap) {
-    ICF_TRY_RC(grow(ctx, &W.tinv, 12LL * n));
-    W.tinv_cap = n;
+    ICF_TRY_RC(icf_grow(ctx, &W.tinv_cap, n, icf_of(&W.tinv, 12LL * n)));
   }
   if (ns + 1LL > W.kcap) {
-    ICF_TRY_RC(grow(ctx, &W.kcnt, ns + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.koff, ns + 1LL));
-    ICF_TRY_RC(grow(ctx, &W.kcur, ns + 1LL));
-    W.kcap = ns + 1LL;
+    ICF_TRY_RC(icf_grow(ctx, &W.kcap, ns + 1LL, &W.kcnt, &W.koff, &W.kcur));
   }
   if (!W.tmpv) ICF_TRY_RC(grow(ctx, &W.tmpv, 8LL * (2 * ctx->n_sm + 1)));
   if (!W.red) ICF_TRY_RC(grow(ctx, &W.red, 8));
@@ -835,18 +802,13 @@ int icf_detect_contacts_impl(icf_ctx *ctx, double pad, const int *d_group, int *
   if (!W.h_gp) ICF_CUDA(ctx, cudaMallocHost(&W.h_gp, 8 * sizeof(int)));
   if (W.cell_cap == 0) {  // a first guess: a cell per surface element
     const long long c = n + 4096LL;
-    ICF_TRY_RC(grow(ctx, &W.gcnt, c));
-    ICF_TRY_RC(grow(ctx, &W.goff, c));
-    ICF_TRY_RC(grow(ctx, &W.gcur, c));
+    ICF_TRY_RC(icf_grow(ctx, &W.cell_cap, c, &W.gcnt, &W.goff, &W.gcur));
     // counts past a call's C are scanned but never read; start them at zero
     ICF_CUDA(ctx, cudaMemsetAsync(W.gcnt, 0, sizeof(int) * (size_t)c, ctx->stream));
-    W.cell_cap = c;
   }
   if (W.nkey_cap == 0) {
     const long long c = std::max<long long>(n / 4, 1024);
-    ICF_TRY_RC(grow(ctx, &W.nk0, c));
-    ICF_TRY_RC(grow(ctx, &W.nk1, c));
-    W.nkey_cap = c;
+    ICF_TRY_RC(icf_grow(ctx, &W.nkey_cap, c, &W.nk0, &W.nk1));
   }
   for (int attempt = 0; attempt < 3; attempt++) {
     bool again = false;

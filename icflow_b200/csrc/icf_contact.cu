@@ -208,14 +208,6 @@ int icf_launch_imp_unit(icf_ctx *ctx, cudaStream_t stream) {
 // result); the buffers are the context's workspace.  The new list is also
 // compared, on the device, with the list the current structure was built
 // from, so that the structure request that follows needs no round trip.
-template <typename T>
-static int grow_buf(icf_ctx *ctx, T **p, long long n) {
-  cudaFree(*p);
-  *p = nullptr;
-  ICF_CUDA(ctx, cudaMalloc(p, sizeof(T) * (size_t)(n > 0 ? n : 1)));
-  return ICF_OK;
-}
-
 int icf_run_narrow_phase(icf_ctx *ctx, int n_pairs, int *n_impacts) {
   cudaStream_t s = ctx->stream;
   icf_contact_ws &W = ctx->cws;
@@ -228,9 +220,7 @@ int icf_run_narrow_phase(icf_ctx *ctx, int n_pairs, int *n_impacts) {
   if (!W.d_small) ICF_CUDA(ctx, cudaMalloc(&W.d_small, 8 * sizeof(int)));
   if (!W.h_small) ICF_CUDA(ctx, cudaMallocHost(&W.h_small, 8 * sizeof(int)));
   if (n_pairs + 1LL > W.ncnt_cap) {
-    ICF_TRY_RC(grow_buf(ctx, &W.ncnt, n_pairs + 1LL));
-    ICF_TRY_RC(grow_buf(ctx, &W.noff, n_pairs + 1LL));
-    W.ncnt_cap = n_pairs + 1LL;
+    ICF_TRY_RC(icf_grow(ctx, &W.ncnt_cap, n_pairs + 1LL, &W.ncnt, &W.noff));
   }
   // counts and offsets of the set bits
   k_narrow<<<icf_blocks(n_pairs, 128), 128, 0, s>>>(n_pairs, ctx->d_pairs, ctx->d_selem, ctx->d_xc,
@@ -250,9 +240,7 @@ int icf_run_narrow_phase(icf_ctx *ctx, int n_pairs, int *n_impacts) {
   if (total > 0) {
     if (total > W.nkey_cap) {
       const long long c = total + total / 4 + 64;
-      ICF_TRY_RC(grow_buf(ctx, &W.nk0, c));
-      ICF_TRY_RC(grow_buf(ctx, &W.nk1, c));
-      W.nkey_cap = c;
+      ICF_TRY_RC(icf_grow(ctx, &W.nkey_cap, c, &W.nk0, &W.nk1));
     }
     // keys node << eb | element, over the bits the ids need
     k_expand<<<icf_blocks(n_pairs, 128), 128, 0, s>>>(n_pairs, ctx->d_pairs, ctx->d_selem, ctx->d_masks, W.noff,
@@ -281,9 +269,8 @@ int icf_finish_impacts(icf_ctx *ctx, const unsigned long long *keys, int total, 
   if (total > 0) {
     // the impact list holds at most `total` entries
     if (total > ctx->imp_cap) {
-      ICF_TRY_RC(grow_buf(ctx, &ctx->d_imp, 2LL * total));
-      ctx->imp_cap = 2 * total;
       ctx->imp_gen++;
+      ICF_TRY_RC(icf_grow(ctx, &ctx->imp_cap, 2LL * total, &ctx->d_imp));
     }
     k_closest<<<icf_blocks(8LL * total, 128), 128, 0, s>>>(total, d_n, eb, keys, ctx->d_adj_off, ctx->d_adj,
                                                           ctx->d_faces, ctx->d_xc, ctx->d_imp);

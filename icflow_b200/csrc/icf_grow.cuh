@@ -5,18 +5,34 @@
 #pragma once
 #include <cstddef>
 
-// Arrays of n elements each in place of the ones at *p, whose contents are not
-// kept.  The capacity holds for all of them: it is zero from the first release
+// an array and its elements
+template <class T>
+struct icf_array {
+  T **p;
+  long long n;
+};
+template <class T>
+icf_array<T> icf_of(T **p, long long n) {
+  return {p, n};
+}
+
+// New arrays in place of the ones at a.p, whose contents are not kept, for a
+// capacity of c.  It holds for all of them: it is zero from the first release
 // until the last allocation has succeeded, so that after a failure the next call
 // allocates all of them again, however few elements it needs.
 template <class Mem, class Cap, class... T>
-bool icf_grow_all(Mem &mem, Cap *cap, long long n, T **...p) {
+bool icf_grow_all(Mem &mem, Cap *cap, long long c, icf_array<T>... a) {
   *cap = 0;
-  ((mem.free(*p), *p = nullptr), ...);
+  ((mem.free(*a.p), *a.p = nullptr), ...);
   bool ok = true;
-  ((ok = ok && mem.alloc(reinterpret_cast<void **>(p), sizeof(T) * (size_t)n)), ...);
-  if (ok) *cap = (Cap)n;
+  ((ok = ok && mem.alloc(reinterpret_cast<void **>(a.p), sizeof(T) * (size_t)a.n)), ...);
+  if (ok) *cap = (Cap)c;
   return ok;
+}
+// of c elements each
+template <class Mem, class Cap, class... T>
+bool icf_grow_all(Mem &mem, Cap *cap, long long c, T **...p) {
+  return icf_grow_all(mem, cap, c, icf_array<T>{p, c}...);
 }
 
 // Temporaries: alloc() registers what it gave, the destructor frees it.

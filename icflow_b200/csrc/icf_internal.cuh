@@ -530,11 +530,11 @@ struct icf_stream_mem {
   }
   void free(void *p) { cudaFreeAsync(p, s); }
 };
-// n elements for each of the arrays that share the capacity *cap
-template <class Cap, class... T>
-int icf_grow(icf_ctx *ctx, Cap *cap, long long n, T **...p) {
+// new arrays (pointers, or icf_of a number of elements) for the capacity n that they share
+template <class Cap, class... A>
+int icf_grow(icf_ctx *ctx, Cap *cap, long long n, A... a) {
   icf_device_mem mem;
-  if (icf_grow_all(mem, cap, n, p...)) return ICF_OK;
+  if (icf_grow_all(mem, cap, n, a...)) return ICF_OK;
   return icf_fail(ctx, ICF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(mem.err));
 }
 #define ICF_TRY_RC(call)        \

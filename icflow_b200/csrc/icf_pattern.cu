@@ -860,18 +860,10 @@ static int build_sell(icf_ctx *ctx, const int4 *desc, int n, int wl, bool with_r
   S->n_real = 0;
   if (n == 0) return ICF_OK;
   const int ns = S->n_slices;
-  if (ns > S->slices_cap || !S->meta) {
-    cudaFree(S->meta);
-    cudaFree(S->unit);
-    cudaFree(S->unit_s);
-    S->unit_s = nullptr;
-    S->meta = nullptr;
-    S->unit = nullptr;
-    const int cap = ns + ns / 4 + 16;
-    ICF_CUDA(ctx, cudaMalloc(&S->meta, sizeof(int4) * (size_t)cap));
-    ICF_CUDA(ctx, cudaMalloc(&S->unit, sizeof(int2) * (size_t)cap * per));
-    ICF_CUDA(ctx, cudaMalloc(&S->unit_s, sizeof(int2) * (size_t)cap * per));
-    S->slices_cap = cap;
+  if (ns > S->slices_cap) {
+    const long long cap = ns + ns / 4 + 16;
+    ICF_TRY_RC(icf_grow(ctx, &S->slices_cap, cap, icf_of(&S->meta, cap), icf_of(&S->unit, cap * per),
+                        icf_of(&S->unit_s, cap * per)));
   }
   uint32_t *k0, *k1;
   int *i0, *perm, *cnt, *off;

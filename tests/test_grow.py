@@ -68,6 +68,10 @@ int main() {
     CHECK(have(1000) && cap == 1000);
     int small_cap = 7;
     CHECK(icf_grow_all(m, &small_cap, 50, &a) && small_cap == 50);
+    m.fail_at = fail < 0 ? -1 : m.calls + fail;
+    CHECK(icf_grow_all(m, &cap, 20, icf_of(&a, 60), icf_of(&b, 21), icf_of(&c, 20)) == (fail < 0));
+    if (fail >= 0) CHECK(cap == 0);
+    if (fail < 0) CHECK(cap == 20 && m.live[a] == 60 * sizeof(int) && m.live[b] == 21 * sizeof(double) && m.live[c] == 20);
   }
   for (int n = 0; n <= 9; n++)
     for (int fail = -1; fail < n; fail++) {
@@ -91,17 +95,18 @@ def test_failed_allocations(tmp_path):
     assert out.returncode == 0, out.stdout
 
 
-CAPS = {"icf_pattern.cu": "rows_cap|items_cap|cols_cap|cr_cap|ks_cap|imp_pos_cap|s2m_cap|rhs_cap",
-        "icf_solve.cu": "[a-z]+_cap"}
+CAPS = {"icf_pattern.cu": "rows_cap|items_cap|cols_cap|cr_cap|ks_cap|imp_pos_cap|s2m_cap|rhs_cap|slices_cap",
+        "icf_solve.cu": "[a-z]+_cap", "icf_broad.cu": r"k?cap|\w+_cap", "icf_contact.cu": r"\w+_cap",
+        "icf_api.cu": "pairs_cap|imp_cap|imp_built_cap"}
 
 
 @pytest.mark.parametrize("name", sorted(CAPS))
 def test_arrays_of_one_capacity_grow_together(name):
-    """The capacities of the structure's merge and of the solver are set by the
-    growth of their arrays, never by hand."""
+    """The capacities of the contact buffers, of the structure's merge and of the
+    solver are set by the growth of their arrays, never by hand (but to zero)."""
     text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
-    text = re.sub(r"\bhalo_cap\b", "", text)  # (a size, not a capacity)
-    assert not re.findall(rf"\b(?:{CAPS[name]})\s*=[^=]", text)
+    text = re.sub(r"const long long c\w* =|\b(?:halo_cap|cap_cells)\b", "", text)  # (sizes, not capacities)
+    assert not re.findall(rf"\b(?:{CAPS[name]})\s*=(?![=]| 0;)[^;]*", text)
 
 
 def test_solver_allocates_by_capacity():
